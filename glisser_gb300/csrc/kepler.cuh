@@ -222,33 +222,54 @@ __device__ __forceinline__ double starter_classic(double dt, double r0, double r
 
 // FP32 pre-solve of the elliptic Kepler equation in the difference form
 //   x - ec sin x + es (1 - cos x) = dM,   s = x / sqrt(alpha)
-// (ec = 1 - r0 alpha/mu, es = u sqrt(alpha)/mu).  Runs on the FP32 pipes; its
-// ~1e-6 relative accuracy only has to put the FP64 iteration in its
-// quartic basin.
+// (ec = 1 - r0 alpha/mu, es = u sqrt(alpha)/mu).  Its ~1e-6 relative accuracy
+// only has to put the FP64 iteration in its quartic basin.
+// Danby's starter for the difference equation, then Halley steps (cubic: two
+// or three from it) until one no longer moves x.
+__device__ __forceinline__ float solve_kepler_f32(float dM, float ec, float es)
+{
+    float sM, cM;
+    __sincosf(dM, &sM, &cM);
+    float x = dM - es + es * cM + ec * sM;
+    for (int k = 0; k < 6; k++) {
+        float sx, cx;
+        sincosf(x, &sx, &cx);
+        const float f = x - ec * sx + es * (1.0f - cx) - dM;
+        const float fp = 1.0f - ec * cx + es * sx;
+        const float fpp = ec * sx + es * cx;
+        float dx = -__fdividef(f, fp);
+        dx = -__fdividef(f, fp + 0.5f * dx * fpp);
+        x += dx;
+        if (fabsf(dx) <= 3e-7f * fabsf(x)) break;
+    }
+    return x;
+}
+
+// The step's mean anomaly below this many radians is formed in FP32 too; a
+// longer step sheds whole turns in FP64 first.
+constexpr float PRESOLVE_F32_DM_MAX = 8.0f;
+
+// The coefficients in FP32 from integer-pipe casts and FP32 square roots and
+// quotients: no FP64 instruction.  Formed in FP64 they took ~70 (a square
+// root, five quotients, a floor) of the ~115 of a drift outside the series
+// starter's domain.  alpha^1.5 outside a float's normal range, or a step of
+// PRESOLVE_F32_DM_MAX or more, takes the FP64 coefficients.
 __device__ __forceinline__ double starter_fp32_kepler(double dt, double r0, double mu, double alpha, double u)
 {
+    const float af = f32_trunc(alpha), muf = f32_trunc(mu), saf = sqrtf(af), a32 = af * saf;
+    const float dMf = __fdividef(a32 * f32_trunc(dt), muf);
+    if (a32 > 1e-30f && muf < 1e30f && dMf > 1e-6f && dMf < PRESOLVE_F32_DM_MAX) {
+        const float rmu = __fdividef(1.0f, muf);
+        const float ec = fmaf(-f32_trunc(r0) * rmu, af, 1.0f), es = f32_trunc(u) * rmu * saf;
+        return f64_of_f32(__fdividef(solve_kepler_f32(dMf, ec, es), saf));
+    }
     double sa = sqrt(alpha);
     double n = alpha * sa / mu;                       // mean motion
     const double two_pi = 6.283185307179586;
     double dM = n * dt;
     double turns = floor(dM / two_pi);
-    float dMf = (float)(dM - turns * two_pi);
-    float ec = (float)(1.0 - r0 * alpha / mu);
-    float es = (float)(u * sa / mu);
-    // Danby's starter for the difference equation
-    float sM, cM;
-    __sincosf(dMf, &sM, &cM);
-    float x = dMf - es + es * cM + ec * sM;
-    for (int k = 0; k < 6; k++) {
-        float sx, cx;
-        sincosf(x, &sx, &cx);
-        float f = x - ec * sx + es * (1.0f - cx) - dMf;
-        float fp = 1.0f - ec * cx + es * sx;
-        float fpp = ec * sx + es * cx;
-        float dx = -f / fp;
-        dx = -f / (fp + 0.5f * dx * fpp);
-        x += dx;
-    }
+    const float x = solve_kepler_f32((float)(dM - turns * two_pi), (float)(1.0 - r0 * alpha / mu),
+                                     (float)(u * sa / mu));
     return ((double)x + turns * two_pi) / sa;
 }
 
