@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(CTA, (LEARNED ? GLISSER_BATCHED_THREADS_PER_SM
         const uint32_t it = sh.item;
         if (it >= total || sh.abort) break;
         const BatchItem w = items[it];
-        load_planet_constants(sh, p.npl, sys.m + (size_t)w.system * p.npl, sys.rh + (size_t)w.system * p.npl,
+        load_planet_constants(p, sh, p.npl, sys.m + (size_t)w.system * p.npl, sys.rh + (size_t)w.system * p.npl,
                               sys.id + (size_t)w.system * p.npl);
         __syncthreads();
         bool ok = run_tile<NP, CTA, PPT, LEARNED, KICK64>(p, sys.log + (size_t)w.system * sys.log_stride, w.first,

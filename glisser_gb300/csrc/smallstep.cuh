@@ -1,0 +1,274 @@
+// Small-step Kepler drift in float-float (FP32 pipe).
+//
+// A drift whose step is a small part of the local dynamical time
+// (tau^2 = dt^2 mu / r0^3 < SMALL_DRIFT_TAU2) moves the particle by
+//   r' = r + dt v + ((f - 1) r + (g - dt) v),
+//   v' = v + (fd r + (gd - 1) v),
+// where f - 1, gd - 1 ~ tau^2 / 2, g / dt - 1 ~ tau^2 / 6 and fd r ~ tau v are
+// small next to what they are added to, so the ~47 bits of a float-float reach
+// past the double's last place.  GB300 issues FP64 at 1/64 of the FP32 rate:
+// the corrections are formed on the FP32 pipe and twelve FP64 instructions
+// remain in a step (dt v, the sums into r and v, |r'|^2), where the general
+// drift (kepler.cuh) and kick execute 44.
+//
+// Kepler's equation, dimensionless.  With s = (dt/r0)(1 + w), X = u dt/(2 r0^2)
+// (u = r.v), A = alpha dt^2/r0^2, Y = (tau^2 - A)/6:
+//   R(w) = w + X (1+w)^2 2c2(x) + Y (1+w)^3 6c3(x) = 0,   x = A (1+w)^2,
+// from r0 G1 + u G2 + mu G3 = dt.  Every term is a correction of the size of
+// w itself (~ e tau / 2).  w starts from the fourth-order reversion, takes one
+// FP32 Newton step (to ~1e-9) and one whose residual R is float-float: what is
+// left is quadratic in 1e-9.  Then, with 1 + q2 = (1+w)^2 2c2 and
+// 1 + q3 = (1+w)^3 6c3,
+//   f - 1  = -H / r0,   gd - 1 = -H / r',   H = mu G2 = (mu dt^2/2r0^2)(1 + q2),
+//   g / dt = 1 - p,     p = (tau^2 / 6)(1 + q3),
+//   fd     = -mu G1 / (r0 r'),  G1 r0 / dt = 1 - X (1 + q2) - p  by Kepler's
+//            equation itself: fd needs ~2^-46, and this form multiplies the
+//            errors of q2 and q3 by X and tau^2 / 6.
+//
+// Bound: issue (about 1,250 FP32 and integer instructions a step with four
+// planets, ~10 cycles of the 128 lanes; twelve FP64 instructions are 6 cycles of
+// the FP64 pipe).  The line at tau^2 = 1e-3: up to there the error of a drift is that of FP64
+// (position 6e-17 rms of |r| against 6e-17, velocity 5e-17 to 1.4e-16 of |v|
+// against 7e-17 for the coefficients correctly rounded); at 1e-3..2e-3 it is
+// 3.4e-16.  Measured on GB300, before (every drift general) and after: 1e6
+// particles x 1,024 steps with four giants 98.6 -> 48.6 ms; 2e6 planet crossers
+// x 100 steps 16.6 -> 6.0 ms; 2,000 particles x 128 steps 643 -> 358 us;
+// 256 ensembles, 1.5e6 particles x 512 steps, 80 -> 44.6 ms.  Position error of
+// those blocks against long double: giants 1.49e-14 -> 1.01e-14 rms, belt
+// 2.34e-14 -> 1.64e-14, crossers 8.6e-16 -> 7.2e-16, scattered disk
+// 3.5e-15 -> 3.0e-15.
+#pragma once
+#include "fastmath.cuh"
+
+namespace glisser {
+
+// Bound on tau^2 of the small-step drift.
+#ifndef GLISSER_SMALL_DRIFT_TAU2
+#define GLISSER_SMALL_DRIFT_TAU2 1e-3f
+#endif
+constexpr float SMALL_DRIFT_TAU2 = GLISSER_SMALL_DRIFT_TAU2;
+
+// --- float-float without the renormalising step: hi + lo with |lo| up to a
+// few units in hi's last place.  Sums and products of them lose ~2^-46; a
+// result is renormalised (ff_norm) where a longer chain follows.
+__device__ __forceinline__ ff ff_norm(ff a) { return ff_fast_two_sum(a.hi, a.lo); }
+
+__device__ __forceinline__ ff ff_mul_u(ff a, ff b)
+{
+    const float p = __fmul_rn(a.hi, b.hi);
+    float e = __fmaf_rn(a.hi, b.hi, -p);
+    e = __fmaf_rn(a.hi, b.lo, e);
+    return { p, __fmaf_rn(a.lo, b.hi, e) };
+}
+
+__device__ __forceinline__ ff ff_sqr_u(ff a)
+{
+    const float p = __fmul_rn(a.hi, a.hi);
+    const float e = __fmaf_rn(a.hi, a.hi, -p);
+    return { p, __fmaf_rn(__fadd_rn(a.hi, a.hi), a.lo, e) };
+}
+
+__device__ __forceinline__ ff ff_add_u(ff a, ff b)
+{
+    const ff s = ff_two_sum(a.hi, b.hi);
+    return { s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)) };
+}
+
+// a . b and |a|^2 of 3-vectors, renormalised
+__device__ __forceinline__ ff ff_sum3(ff p, ff q, ff r)
+{
+    const ff s = ff_two_sum(p.hi, q.hi);
+    const ff t = ff_two_sum(s.hi, r.hi);
+    return ff_fast_two_sum(t.hi, __fadd_rn(__fadd_rn(s.lo, t.lo), __fadd_rn(__fadd_rn(p.lo, q.lo), r.lo)));
+}
+
+__device__ __forceinline__ ff ff_dot3(ff ax, ff ay, ff az, ff bx, ff by, ff bz)
+{
+    return ff_sum3(ff_mul_u(ax, bx), ff_mul_u(ay, by), ff_mul_u(az, bz));
+}
+
+__device__ __forceinline__ ff ff_sqr3(ff x, ff y, ff z) { return ff_sum3(ff_sqr_u(x), ff_sqr_u(y), ff_sqr_u(z)); }
+
+// The rare halves of ff_split_fast and ff_widen, as calls: inlined, the compiler
+// turns their branches into predicated instructions that every step issues
+// (ff_widen's FP64 conversions and addition, so issued, made the crossers'
+// block 1.9x longer).
+static __device__ __noinline__ ff ff_split_rare(double d) { return ff_split(d); }
+static __device__ __noinline__ double ff_widen_rare(float hi, float lo) { return (double)hi + (double)lo; }
+
+// A double as a float-float on the integer and FP32 pipes: hi = d rounded to
+// 24 significant bits, lo = the (signed) rest rounded to 24: |d - hi - lo| <
+// 2^-49 |d|, for |d| < 2^127.  ff_split counts leading zeros to place lo; here
+// the conversion instruction does.  Zero and |d| < 2^-70 (where lo's unit would
+// leave the float range) take ff_split.
+__device__ __forceinline__ ff ff_split_fast(double d)
+{
+    const unsigned hw = (unsigned)__double2hiint(d), lw = (unsigned)__double2loint(d);
+    if ((hw & 0x7fffffffu) < ((1023u - 70u) << 20)) return ff_split_rare(d);
+    // exponent and top 23 significand bits in a float's places; rebiasing from
+    // 1023 to 127 adds -896 << 23, 0x40000000 modulo 2^32; bit 28 rounds
+    const unsigned f = __funnelshift_l(lw, hw, 3);
+    const unsigned h = ((f + 0x40000000u + ((lw >> 28) & 1u)) & 0x7fffffffu) | (hw & 0x80000000u);
+    // the rest: the low 29 bits, signed, in units of 2^(e - 52); as the top of a
+    // 32-bit integer in units of 2^(e - 55), with d's sign
+    const float rest = (float)(int)(lw << 3);
+    const unsigned unit = (((f & 0x7f800000u) + (0x40000000u - (55u << 23))) & 0x7fffffffu) | (hw & 0x80000000u);
+    return { __uint_as_float(h), __fmul_rn(rest, __uint_as_float(unit)) };
+}
+
+// hi + lo as a double on the integer and FP32 pipes, to ~2^-47 of it (lo
+// enters in units of 2^-46 of hi's binade), for a renormalised pair: hi widened
+// exactly, lo's multiple of the unit added to the magnitude bits.  hi a power
+// of two (the sum may fall into the binade below, whose unit is another), zero
+// or below 2^-76 takes the FP64 addition.
+__device__ __forceinline__ double ff_widen(ff x)
+{
+    const unsigned b = __float_as_uint(x.hi), m = b & 0x7fffffffu;
+    if ((b & 0x007fffffu) == 0u || m < ((127u - 76u) << 23)) return ff_widen_rare(x.hi, x.lo);
+    // 2^(46 - e) with hi's sign, so that the multiple is relative to hi's; the
+    // FMA rounds it to an integer in the last places of 1.5 * 2^23
+    const float scale = __uint_as_float(((127u + 46u + 127u) << 23) - (b & 0xff800000u));
+    const int k = __float_as_int(__fmaf_rn(x.lo, scale, 12582912.0f)) - 0x4b400000;
+    const unsigned hw = (m >> 3) + ((1023u - 127u) << 20) + (b & 0x80000000u);
+    return __longlong_as_double((long long)((unsigned long long)hw << 32 | (b << 29)) + ((long long)k << 6));
+}
+
+// 1/x by the special-function unit (~1 unit in the last place)
+__device__ __forceinline__ float rcp_approx(float x)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / x;
+#endif
+}
+
+// e = 1 - x y^2 for the seed y of 1/sqrt(x): the product's leading part cancels
+// against 1 inside the first FMA, so each of the three roundings is of a
+// number of e's own size (2^-22), below 2^-47
+__device__ __forceinline__ float rsqrt_residual(ff x, float y)
+{
+    const ff y2 = ff_two_prod(y, y);
+    return __fmaf_rn(-x.lo, y2.hi, __fmaf_rn(-x.hi, y2.lo, __fmaf_rn(-x.hi, y2.hi, 1.0f)));
+}
+
+// 1/sqrt(x) of a float-float, to ~2^-48: y (1 + e/2 + 3e^2/8) with e = 1 - x y^2 as
+// a float-float (1 - x.hi y^2.hi is exact, the rest some 2^-24) and y e/2 as an
+// exact product
+__device__ __forceinline__ ff ff_rsqrt(ff x)
+{
+    const float y = rsqrtf(x.hi), h = 0.5f * y;
+    const ff y2 = ff_two_prod(y, y), t = ff_two_prod(x.hi, y2.hi);
+    const ff e = ff_two_sum(__fsub_rn(1.0f, t.hi), -__fmaf_rn(x.lo, y2.hi, __fmaf_rn(x.hi, y2.lo, t.lo)));
+    const ff d = ff_two_prod(h, e.hi);
+    const ff s = ff_fast_two_sum(y, d.hi);
+    return { s.hi, __fadd_rn(s.lo, __fmaf_rn(h, __fmaf_rn(0.75f * e.hi, e.hi, e.lo), d.lo)) };
+}
+
+// 1/x of a float-float, the same way: y (1 + e + e^2), e = 1 - x y
+__device__ __forceinline__ ff ff_rcp(ff x)
+{
+    const float y = rcp_approx(x.hi);
+    const ff t = ff_two_prod(x.hi, y);
+    const ff e = ff_two_sum(__fsub_rn(1.0f, t.hi), -__fmaf_rn(x.lo, y, t.lo));
+    const ff d = ff_two_prod(y, e.hi);
+    const ff s = ff_fast_two_sum(y, d.hi);
+    return { s.hi, __fadd_rn(s.lo, __fmaf_rn(y, __fmaf_rn(e.hi, e.hi, e.lo), d.lo)) };
+}
+
+// Constants of a launch's step dt.
+struct SmallStepDt {
+    ff dt2, dt_half, neg_dt;      // dt^2, dt / 2, -dt
+};
+
+// A drift's coefficients: f - 1, g - dt, H (gd - 1 = -H / r') and fd r'.
+struct SmallDrift {
+    ff f1, gdt, h, fdr;
+};
+
+// The coefficients of one drift from the float-float split of its state, of r0^2
+// and 1/r0 (muh = mu dt^2 / 2, mudt = mu dt).  False outside the small-step domain
+// -- tau^2 at or above SMALL_DRIFT_TAU2, not bound beyond the energy's rounding,
+// or a value outside the range that float-float covers (a NaN in 1/r0 says so).
+// The decision is each particle's own, so that its path does not depend on the
+// particles that share its warp.
+__device__ __forceinline__ bool small_drift(ff rx, ff ry, ff rz, ff vx, ff vy, ff vz, ff r2, ff rinv,
+                                            ff muh, ff mudt, const SmallStepDt& c, SmallDrift& d)
+{
+    const ff u = ff_dot3(rx, ry, rz, vx, vy, vz);
+    const ff v2 = ff_sqr3(vx, vy, vz);
+    // 1/r0^2 from r0^2, not from 1/r0: the square of a float-float drops its lo^2,
+    // below its last place and so never rounded up to it -- a bias of 8e-16 in the
+    // Sun's pull, which adds up over the steps
+    const ff ri2 = ff_rcp(r2);
+    const ff m2 = ff_mul(muh, ri2);                                   // mu dt^2 / (2 r0^2)
+    const ff th = ff_mul(m2, rinv);                                   // tau^2 / 2
+    const ff b = ff_mul(ff_mul_u(c.dt2, ri2), v2);                    // (v dt / r0)^2
+    const ff X = ff_mul(ff_mul_u(c.dt_half, ri2), u);
+    // A = 2 tau^2 - b and 6 Y = tau^2 - A = b - tau^2
+    const ff A = ff_add_u(ff_scale(th, 4.0f), ff_neg(b));
+    const ff Y = ff_mul_u(ff_add_u(b, ff_scale(th, -2.0f)), ff_sixth());
+    const float a = A.hi, x = X.hi, y = Y.hi;
+    const bool inside = th.hi < 0.5f * SMALL_DRIFT_TAU2 && th.hi > 0x1p-30f && a > 0x1p-20f * th.hi;
+    if (!inside) return false;
+
+    // FP32: fourth-order start and one Newton step,
+    // R' = 1 + 2X (1+w) c1(x) + 3Y (1+w)^2 2c2(x)
+    float w = __fmaf_rn(x, __fmaf_rn(a, 1.0f / 12.0f, __fmaf_rn(__fmaf_rn(-5.0f, x, 2.0f), x, __fmaf_rn(5.0f, y, -1.0f))), -y);
+    float s = 1.0f + w, s2 = s * s, xx = a * s2;
+    const float rp = rcp_approx(__fmaf_rn(2.0f * x * s, __fmaf_rn(xx, -1.0f / 6.0f, 1.0f),
+                                          __fmaf_rn(3.0f * y * s2, __fmaf_rn(xx, -1.0f / 12.0f, 1.0f), 1.0f)));
+    const float res = __fmaf_rn(x * s2, __fmaf_rn(xx, __fmaf_rn(xx, 1.0f / 360.0f, -1.0f / 12.0f), 1.0f),
+                                __fmaf_rn(y * s2 * s, __fmaf_rn(xx, -1.0f / 20.0f, 1.0f), w));
+    w = __fmaf_rn(-res, rp, w);
+
+    // with z = (1+w)^2 - 1:
+    // q2 = z - (A/12) (1 + 2z) + [ -(A/12) z^2 + A^2/360 (1+w)^6 - A^3/20160 (1+w)^8 ],
+    // q3 = 3w + 3w^2 + [ w^3 + (1+w)^3 (6c3 - 1) ], the brackets in FP32
+    const ff ww = ff_two_prod(w, w), A12 = ff_mul_u(A, ff_twelfth());
+    ff z = ff_fast_two_sum(2.0f * w, ww.hi);
+    z.lo += ww.lo;
+    s = 1.0f + w;
+    s2 = 1.0f + z.hi;
+    xx = a * s2;
+    const ff az = ff_mul_u(A12, ff_scale(z, 2.0f));
+    const float rest2 = __fmaf_rn(-A12.hi * z.hi, z.hi,
+                                  s2 * xx * xx * __fmaf_rn(xx, -1.0f / 20160.0f, 1.0f / 360.0f));
+    const ff t1 = ff_two_sum(z.hi, -A12.hi);
+    const ff t2 = ff_fast_two_sum(t1.hi, -az.hi);
+    ff q2 = { t2.hi, __fadd_rn(__fadd_rn(__fadd_rn(t1.lo, t2.lo), __fsub_rn(z.lo, A12.lo)), __fsub_rn(rest2, az.lo)) };
+    const float w3 = 3.0f * w, ww3 = 3.0f * ww.hi;
+    ff q3 = ff_fast_two_sum(w3, ww3);
+    q3.lo = (q3.lo + (__fmaf_rn(3.0f, w, -w3) + __fmaf_rn(3.0f, ww.hi, -ww3))) +
+            __fmaf_rn(ww.hi, w, s2 * s * xx * __fmaf_rn(xx, __fmaf_rn(xx, -1.0f / 60480.0f, 1.0f / 840.0f),
+                                                       -1.0f / 20.0f));
+    // R = w + X + X q2 + Y + Y q3 and the second Newton step
+    const ff xq = ff_mul_u(X, q2);
+    const ff e1 = ff_two_sum(x, w);
+    const ff e2 = ff_two_sum(e1.hi, xq.hi);
+    const ff yq = ff_mul_u(Y, q3);
+    const ff e3 = ff_two_sum(e2.hi, y);
+    const float lows = __fadd_rn(__fadd_rn(__fadd_rn(e1.lo, e2.lo), __fadd_rn(e3.lo, xq.lo)),
+                                 __fadd_rn(__fadd_rn(X.lo, Y.lo), yq.lo));
+    const float dw = -__fadd_rn(__fadd_rn(e3.hi, yq.hi), lows) * rp;
+    q2.lo = __fmaf_rn(2.0f * s, dw, q2.lo);
+    q3.lo = __fmaf_rn(3.0f * s2, dw, q3.lo);
+
+    const ff o2 = ff_fast_two_sum(1.0f, q2.hi), o3 = ff_fast_two_sum(1.0f, q3.hi);
+    d.h = ff_mul(m2, ff{ o2.hi, o2.lo + q2.lo });
+    d.f1 = ff_neg(ff_mul_u(d.h, rinv));
+    const ff p = ff_mul(ff_mul_u(th, ff_third()), ff{ o3.hi, o3.lo + q3.lo });
+    d.gdt = ff_mul_u(c.neg_dt, p);
+    // fd r' = -(mu dt / r0^2) (1 - X - X q2 - p)
+    const ff xs = ff_two_sum(x, xq.hi);
+    const ff ps = ff_two_sum(xs.hi, p.hi);
+    const float el = __fadd_rn(__fadd_rn(xs.lo, ps.lo),
+                               __fadd_rn(__fadd_rn(X.lo, xq.lo), __fmaf_rn(2.0f * s * x, dw, p.lo)));
+    const ff os = ff_fast_two_sum(1.0f, -ps.hi);
+    d.fdr = ff_mul(ff_neg(ff_mul_u(mudt, ri2)), ff{ os.hi, __fsub_rn(os.lo, el) });
+    return true;
+}
+
+}  // namespace glisser

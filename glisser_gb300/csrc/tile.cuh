@@ -2,7 +2,10 @@
 // kernels (see timeblock.cu for the design).  Header-only: every function is
 // device inline or host inline, compiled into each kernel translation unit.
 #pragma once
+#include <cmath>
+
 #include "kepler.cuh"
+#include "smallstep.cuh"
 #include "timeblock.cuh"
 
 namespace glisser {
@@ -14,8 +17,12 @@ struct Common {
     uint32_t len;
     uint32_t chunk;
     double dt;
+    double inv_dt;
     double outer2;
     double tol_dt;          // Kepler residual tolerance x dt
+    SmallStepDt sdt;        // the step's constants of the small-step drift
+    float dt_range;         // dt within the range those constants cover: 1, else NaN (the general drift runs)
+    float r2_hi;            // |r|^2 above which the radius tests and ranges are looked at one by one
     int starter;
     int kill;
     bool kick64;            // GLISSER_KICK_FP64: the FP64-kick kernels
@@ -99,13 +106,14 @@ __device__ __forceinline__ void issue_chunk(const Common& p, const double* log, 
 }
 
 // What the float-float kick reads of planet j, packed in 32 bytes so that a
-// step reads it with two 16-byte shared-memory loads instead of five.
+// step reads it with two 16-byte shared-memory loads; the hot path reads only
+// the first.  Masses carry the factor -dt: the kick sums velocity changes.
 struct __align__(16) PlanetConst {
-    ff m;                       // m and rh^2 as float-floats
-    ff rh2;
-    double m15;                 // 1.5 m, the FP64 planet pull's form (its fallback)
+    ff mdt;                     // -m dt
+    float near2;                // |dr|^2 at or below which the encounter test and the range are looked at
     float rh2win;               // 2^-40 rh^2: the borderline window of the float-float radius test
-    uint32_t id;
+    ff rh2;                     // rh^2
+    double mdt15;               // -1.5 m dt, the FP64 planet pull's form (its fallback)
 };
 
 // Shared-memory state of one CTA.
@@ -114,6 +122,8 @@ struct CtaShared {
     double rh2[MAX_PLANETS];
     uint32_t id[MAX_PLANETS];
     PlanetConst pk[MAX_PLANETS];
+    ff muh, mudt;               // mu dt^2 / 2, mu dt
+    float r2_lo;                // |r|^2 below which the Sun's radius test is looked at
     uint64_t bar[2];
     int abort;
     uint32_t item;
@@ -134,31 +144,49 @@ __device__ __forceinline__ uint32_t near_nonneg(double x, double t)
     return (unsigned long long)(d + 8192) <= 16384ull ? 1u : 0u;
 }
 
-// Pull of planet j, m dr / |dr|^3 with dr = r - r_j, added to the sum s,
-// and its encounter test (src/wh.cu:145-160): the first planet inside its
-// radius wins (flags == 0 guard).  All in float-float on the FP32 pipe (the
-// position r and the staged planet log as float-floats): the planet terms
-// are perturbations next to the Sun's pull, which the drift integrates in
-// FP64, and carry ~1e-13 of their own size.
+// Ranges that the hot path's float-float products cover without under- or
+// overflow: squared distances, and the bound below which m dt may lie.
+constexpr float KICK_R2_MIN = 0x1p-40f, KICK_R2_MAX = 0x1p44f;
+constexpr float KICK_MDT_MIN = 0x1p-40f, KICK_MDT_MAX = 0x1p30f;
+
+// Velocity change by planet j over dt, -m dt dr / |dr|^3 with dr = r - r_j,
+// added to the sum s, and its encounter test (src/wh.cu:145-160): the first
+// planet inside its radius wins (flags == 0 guard).  All in float-float on the
+// FP32 pipe (the position r and the staged planet log as float-floats): the
+// planet terms are perturbations next to the Sun's pull, which the drift
+// integrates, and carry ~1e-13 of their own size.  One comparison keeps the
+// encounter test, its borderline window and the range checks off the hot path:
+// near2 lies 2^-20 of it above rh^2 (infinite for a mass outside the range).
+// The sum is not renormalised: its lo collects the rounding errors of a few
+// terms and is folded in once, at the step's end.
 __device__ __forceinline__ void planet_kick(const ff* L, int j, ff rx, ff ry, ff rz, ff& sx, ff& sy, ff& sz,
                                             uint16_t& flags, uint32_t& border, const CtaShared& sh)
 {
     const ff dx = ff_add(rx, ff_neg(L[3 * j]));
     const ff dy = ff_add(ry, ff_neg(L[3 * j + 1]));
     const ff dz = ff_add(rz, ff_neg(L[3 * j + 2]));
-    const ff rad = ff_add(ff_add(ff_sqr(dx), ff_sqr(dy)), ff_sqr(dz));
-    const PlanetConst q = sh.pk[j];
-    if (flags == 0) {
-        // rad.hi - rh2.hi is exact near the threshold (Sterbenz), so the FP32
-        // difference is good to a few units of the low parts
-        const float d = __fadd_rn(__fsub_rn(rad.hi, q.rh2.hi), __fsub_rn(rad.lo, q.rh2.lo));
-        border += fabsf(d) <= q.rh2win ? 1u : 0u;
-        if (ff_lt(rad, q.rh2)) flags = (uint16_t)((q.id << 8) | 0x0001);
+    const ff rad = ff_sqr3(dx, dy, dz);
+    const PlanetConst& q = sh.pk[j];
+    ff fac;
+    if (rad.hi > q.near2 && rad.hi < KICK_R2_MAX) {
+        // m |dr|^-3 from the seed y: m y^3 (1 + 1.5 e + 1.875 e^2), e = 1 - |dr|^2 y^2
+        const float y = rsqrtf(rad.hi);
+        const float e = rsqrt_residual(rad, y);
+        const ff my3 = ff_mul_u(q.mdt, ff_mul_f(ff_two_prod(y, y), y));
+        fac = ff_fast_two_sum(my3.hi, __fmaf_rn(my3.hi, __fmul_rn(e, __fmaf_rn(1.875f, e, 1.5f)), my3.lo));
+    } else {
+        if (flags == 0) {
+            // rad.hi - rh2.hi is exact near the threshold (Sterbenz), so the FP32
+            // difference is good to a few units of the low parts
+            const float d = __fadd_rn(__fsub_rn(rad.hi, q.rh2.hi), __fsub_rn(rad.lo, q.rh2.lo));
+            border += fabsf(d) <= q.rh2win ? 1u : 0u;
+            if (ff_lt(rad, q.rh2)) flags = (uint16_t)((sh.id[j] << 8) | 0x0001);
+        }
+        fac = pull_factor_ff(rad, q.mdt, q.mdt15);
     }
-    const ff fac = pull_factor_ff(rad, q.m, q.m15);
-    sx = ff_add(sx, ff_mul(dx, fac));
-    sy = ff_add(sy, ff_mul(dy, fac));
-    sz = ff_add(sz, ff_mul(dz, fac));
+    sx = ff_add_u(sx, ff_mul_u(dx, fac));
+    sy = ff_add_u(sy, ff_mul_u(dy, fac));
+    sz = ff_add_u(sz, ff_mul_u(dz, fac));
 }
 
 // The same kick term in FP64, as the reference computes it (src/wh.cu:142-160:
@@ -208,7 +236,13 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
     // the acceleration is not carried between steps: each step's is used at
     // once for the merged kick, and the last one a particle reaches (flagged
     // or at the block's end) is stored at that step
-    double rx[PPT], ry[PPT], rz[PPT], vx[PPT], vy[PPT], vz[PPT], r2[PPT], rinv[PPT];
+    double rx[PPT], ry[PPT], rz[PPT], vx[PPT], vy[PPT], vz[PPT];
+    // the position, |r|^2 and 1/|r| as float-floats, for the small-step drift and the
+    // kick; |r|^2 and 1/|r| in FP64 for the general drift, current only after
+    // a step that took it (`general`)
+    ff fx[PPT], fy[PPT], fz[PPT], f2[PPT], fri[PPT];
+    double r2[PPT], rinv[PPT];
+    bool general[PPT];
     // neither the block-start flags nor the deathtime index are carried:
     // the index is stored at the particle's last step (flagged or the
     // block's end), and the start flags are read back from memory at the end
@@ -233,16 +267,20 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
         // Kick-drift-kick with the two half kicks between consecutive steps
         // merged into one full kick (v += a dt); a particle takes the closing
         // half kick when it is flagged or the block ends, so its stored
-        // velocity is always at a step boundary.  Each drift returns |r|^2 and
-        // 1/|r| of the position it produces: the Sun/outer test's and the next
-        // drift's.
+        // velocity is always at a step boundary.
         if (flags[k] == 0 && p.len > 0) {
             vx[k] = fma(a0x, hdt, vx[k]);
             vy[k] = fma(a0y, hdt, vy[k]);
             vz[k] = fma(a0z, hdt, vz[k]);
         }
-        r2[k] = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
-        rinv[k] = rsqrt_lean(r2[k]);
+        fx[k] = ff_split_fast(rx[k]);
+        fy[k] = ff_split_fast(ry[k]);
+        fz[k] = ff_split_fast(rz[k]);
+        f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
+        fri[k] = ff_rsqrt(f2[k]);
+        if (!(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX)) fri[k].hi = __int_as_float(0x7fc00000);
+        r2[k] = rinv[k] = 0;
+        general[k] = false;
     }
 
     bool ok = true;
@@ -269,8 +307,13 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
         double* Lw = stage + b * bufstride;
         if constexpr (!KICK64) {
             // the chunk's planet log as float-floats, in place (each 8-byte
-            // double becomes the 8-byte pair of floats the kick reads)
-            for (uint32_t i = tid; i < steps * rec; i += CTA) reinterpret_cast<ff*>(Lw)[i] = ff_split(Lw[i]);
+            // double becomes the 8-byte pair of floats the kick reads), h0 as
+            // the velocity change h0 dt
+            for (uint32_t i = tid; i < steps * rec; i += CTA) {
+                double x = Lw[i];
+                if (i % rec < 3u) x *= p.dt;
+                reinterpret_cast<ff*>(Lw)[i] = ff_split_fast(x);
+            }
         }
         __syncthreads();
         for (uint32_t s = 0; s < steps; s++) {
@@ -279,16 +322,68 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
                 if (flags[k] != 0) continue;
-                const DriftInvariants q =
-                    drift_invariants(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], p.dt, mu);
-                DriftResult d = kepler_drift<LEARNED, NET_ROWS, NET_QU>(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k],
-                                                                         rinv[k], q, p.dt, mu, p.starter, p.mlp,
-                                                                         p.tol_dt);
-                uint16_t fl = d.flags;
-                evals += d.evals;
-                if constexpr (LEARNED) nets += d.net;
-                wide += d.wide;
+                uint16_t fl = 0;
+                SmallDrift sd;
+                ff wx, wy, wz;
+                // this step's velocity change beyond vx..vz, summed with the kick's
+                ff gx = { 0.0f, 0.0f }, gy = { 0.0f, 0.0f }, gz = { 0.0f, 0.0f };
+                // tau^2 / 2 in FP32 first: a wide drift costs the small-step one five instructions
+                const float q3 = sh.muh.hi * fri[k].hi * (fri[k].hi * fri[k].hi);
+                bool small = p.starter != STARTER_CLASSIC && q3 < 0.5f * SMALL_DRIFT_TAU2;
+                if (small) {
+                    wx = ff_split_fast(vx[k]);
+                    wy = ff_split_fast(vy[k]);
+                    wz = ff_split_fast(vz[k]);
+                    small = small_drift(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
+                }
+                if (small) {
+                    // r' = r + dt v + ((f - 1) r + (g - dt) v): dt v in FP64, the rest a
+                    // float-float correction
+                    const ff cx = ff_norm(ff_add_u(ff_mul_u(sd.f1, fx[k]), ff_mul_u(sd.gdt, wx)));
+                    const ff cy = ff_norm(ff_add_u(ff_mul_u(sd.f1, fy[k]), ff_mul_u(sd.gdt, wy)));
+                    const ff cz = ff_norm(ff_add_u(ff_mul_u(sd.f1, fz[k]), ff_mul_u(sd.gdt, wz)));
+                    rx[k] += fma(p.dt, vx[k], ff_widen(cx));
+                    ry[k] += fma(p.dt, vy[k], ff_widen(cy));
+                    rz[k] += fma(p.dt, vz[k], ff_widen(cz));
+                    const ff ox = fx[k], oy = fy[k], oz = fz[k];
+                    fx[k] = ff_split_fast(rx[k]);
+                    fy[k] = ff_split_fast(ry[k]);
+                    fz[k] = ff_split_fast(rz[k]);
+                    // |r'|^2 in FP64 (three instructions of a pipe with room), then
+                    // 1/|r'| in float-float
+                    f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
+                    fri[k] = ff_rsqrt(f2[k]);
+                    // v' = v + (fd r + (gd - 1) v)
+                    const ff gd1 = ff_neg(ff_mul_u(sd.h, fri[k]));
+                    const ff fd = ff_mul(sd.fdr, fri[k]);
+                    gx = ff_add_u(ff_mul_u(fd, ox), ff_mul_u(gd1, wx));
+                    gy = ff_add_u(ff_mul_u(fd, oy), ff_mul_u(gd1, wy));
+                    gz = ff_add_u(ff_mul_u(fd, oz), ff_mul_u(gd1, wz));
+                    general[k] = false;
+                    evals++;
+                } else {
+                    if (!general[k]) {
+                        r2[k] = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
+                        rinv[k] = rsqrt_lean(r2[k]);
+                        general[k] = true;
+                    }
+                    const DriftInvariants q =
+                        drift_invariants(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], p.dt, mu);
+                    DriftResult d = kepler_drift<LEARNED, NET_ROWS, NET_QU>(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k],
+                                                                             r2[k], rinv[k], q, p.dt, mu, p.starter,
+                                                                             p.mlp, p.tol_dt);
+                    fl = d.flags;
+                    evals += d.evals;
+                    if constexpr (LEARNED) nets += d.net;
+                    wide += d.wide;
+                    fx[k] = ff_split_fast(rx[k]);
+                    fy[k] = ff_split_fast(ry[k]);
+                    fz[k] = ff_split_fast(rz[k]);
+                    f2[k] = ff_split_fast(r2[k]);
+                    fri[k] = ff_split_fast(rinv[k]);
+                }
                 double aax, aay, aaz;
+                ff sx, sy, sz;
                 if constexpr (KICK64) {
                     aax = Ld[0]; aay = Ld[1]; aaz = Ld[2];
                     if constexpr (NP > 0) {
@@ -300,41 +395,52 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                             planet_kick64(Ld, j, rx[k], ry[k], rz[k], aax, aay, aaz, fl, border, sh);
                     }
                 } else {
-                    const ff fx = ff_split(rx[k]), fy = ff_split(ry[k]), fz = ff_split(rz[k]);
-                    ff sx = { 0.0f, 0.0f }, sy = { 0.0f, 0.0f }, sz = { 0.0f, 0.0f };
-                    // the planet loop stays rolled: the kernel is bound by
+                    // dt (h0 - sum of the planets' pulls).  The planet loop stays rolled: the kernel is bound by
                     // instruction fetch, and the unrolled four-planet
                     // float-float kick measured 9-12 % slower (the ensemble
                     // kernel and the single-system plain-giants kernel)
+                    sx = L[0]; sy = L[1]; sz = L[2];
                     if constexpr (NP > 0) {
 #pragma unroll 1
-                        for (int j = 1; j <= NP; j++) planet_kick(L, j, fx, fy, fz, sx, sy, sz, fl, border, sh);
+                        for (int j = 1; j <= NP; j++) planet_kick(L, j, fx[k], fy[k], fz[k], sx, sy, sz, fl, border, sh);
                     } else {
-                        for (int j = 1; j <= np; j++) planet_kick(L, j, fx, fy, fz, sx, sy, sz, fl, border, sh);
+                        for (int j = 1; j <= np; j++) planet_kick(L, j, fx[k], fy[k], fz[k], sx, sy, sz, fl, border, sh);
                     }
-                    // a = h0 - sum of the planets' pulls, to FP64 on the integer pipe
-                    const ff gx = ff_add(L[0], ff_neg(sx)), gy = ff_add(L[1], ff_neg(sy)),
-                             gz = ff_add(L[2], ff_neg(sz));
-                    aax = ff_to_f64(gx);
-                    aay = ff_to_f64(gy);
-                    aaz = ff_to_f64(gz);
                 }
-                const double rr = r2[k];
-                border += near_nonneg(rr, rh2_sun) + near_nonneg(rr, p.outer2);
-                if (lt_nonneg(rr, rh2_sun)) fl = 0x0001;
-                if (gt_nonneg(rr, p.outer2)) fl = 0x0002;
+                if (!(f2[k].hi > sh.r2_lo && f2[k].hi < p.r2_hi)) {
+                    // near or beyond a radius, or outside the float-float range
+                    const double rr = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
+                    border += near_nonneg(rr, rh2_sun) + near_nonneg(rr, p.outer2);
+                    if (lt_nonneg(rr, rh2_sun)) fl = 0x0001;
+                    if (gt_nonneg(rr, p.outer2)) fl = 0x0002;
+                    if (!(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX)) fri[k].hi = __int_as_float(0x7fc00000);
+                }
                 flags[k] = fl;
                 const uint32_t step = cfirst + s + 1;
                 const bool last = fl != 0 || step == p.len;
                 if (last) {
                     const uint32_t i = first + (uint32_t)k * CTA + tid;
+                    if constexpr (!KICK64) {
+                        aax = ff_to_f64(ff_norm(sx)) * p.inv_dt;
+                        aay = ff_to_f64(ff_norm(sy)) * p.inv_dt;
+                        aaz = ff_to_f64(ff_norm(sz)) * p.inv_dt;
+                        sx = ff_scale(sx, 0.5f);
+                        sy = ff_scale(sy, 0.5f);
+                        sz = ff_scale(sz, 0.5f);
+                    }
                     p.pa.ax[i] = aax; p.pa.ay[i] = aay; p.pa.az[i] = aaz;
                     p.pa.deathtime_index[i] = step;
                 }
-                const double kc = last ? hdt : p.dt;
-                vx[k] = fma(aax, kc, vx[k]);
-                vy[k] = fma(aay, kc, vy[k]);
-                vz[k] = fma(aaz, kc, vz[k]);
+                if constexpr (KICK64) {
+                    const double kc = last ? hdt : p.dt;
+                    vx[k] += fma(aax, kc, ff_widen(ff_norm(gx)));
+                    vy[k] += fma(aay, kc, ff_widen(ff_norm(gy)));
+                    vz[k] += fma(aaz, kc, ff_widen(ff_norm(gz)));
+                } else {
+                    vx[k] += ff_widen(ff_norm(ff_add_u(gx, sx)));
+                    vy[k] += ff_widen(ff_norm(ff_add_u(gy, sy)));
+                    vz[k] += ff_widen(ff_norm(ff_add_u(gz, sz)));
+                }
             }
         }
         __syncthreads();
@@ -424,20 +530,33 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
     return ok;
 }
 
-__device__ __forceinline__ void load_planet_constants(CtaShared& sh, uint32_t npl, const double* m, const double* rh,
-                                                      const uint32_t* pid)
+__device__ __forceinline__ void load_planet_constants(const Common& p, CtaShared& sh, uint32_t npl, const double* m,
+                                                      const double* rh, const uint32_t* pid)
 {
     for (uint32_t j = threadIdx.x; j < npl; j += blockDim.x) {
+        const double rh2 = rh[j] * rh[j];
         sh.m[j] = m[j];
-        sh.rh2[j] = rh[j] * rh[j];
+        sh.rh2[j] = rh2;
         sh.id[j] = pid[j];
+        const double mdt = -m[j] * p.dt;
         PlanetConst q;
-        q.m = ff_split(m[j]);
-        q.rh2 = ff_split(sh.rh2[j]);
-        q.m15 = 1.5 * m[j];
+        q.mdt = ff_split(mdt);
+        q.mdt15 = 1.5 * mdt;
+        q.rh2 = ff_split(rh2);
         q.rh2win = q.rh2.hi * 0x1p-40f;
-        q.id = pid[j];
+        const float near = fmaxf(q.rh2.hi * (1.0f + 0x1p-20f), KICK_R2_MIN);
+        const float am = fabsf(q.mdt.hi);
+        q.near2 = m[j] == 0.0 || (am > KICK_MDT_MIN && am < KICK_MDT_MAX) ? near : __int_as_float(0x7f800000);
         sh.pk[j] = q;
+        if (j == 0) {
+            const double muh = 0.5 * m[0] * p.dt * p.dt;
+            sh.muh = ff_split_fast(muh);
+            sh.mudt = ff_split(-mdt);
+            // outside the range the constant's products cover, NaN: the general drift runs
+            if (!(sh.muh.hi > 0x1p-40f && sh.muh.hi < 0x1p30f)) sh.muh.hi = __int_as_float(0x7fc00000);
+            sh.muh.hi *= p.dt_range;
+            sh.r2_lo = near;
+        }
     }
 }
 
@@ -452,6 +571,12 @@ __device__ __forceinline__ void init_barriers(CtaShared& sh)
 }
 
 
+inline ff ff_of(double d)
+{
+    const float h = (float)d;
+    return { h, (float)(d - (double)h) };
+}
+
 inline bool fill_common(Common& p, const glisser_particles* pa, const glisser_step_params* sp, const glisser_handoff* ho,
                  uint32_t npl, uint32_t len, uint32_t max_chunk = LOG_CHUNK)
 {
@@ -459,7 +584,15 @@ inline bool fill_common(Common& p, const glisser_particles* pa, const glisser_st
     p.npl = npl;
     p.len = len;
     p.dt = sp->dt;
+    p.inv_dt = 1.0 / sp->dt;
     p.outer2 = sp->outer_radius * sp->outer_radius;
+    // one comparison keeps the outer-limit test off the hot path: 2^-20 below
+    // the limit (a limit outside the float range leaves the range's own bound)
+    p.r2_hi = (float)std::fmin(p.outer2 * (1.0 - 0x1p-20), (double)KICK_R2_MAX);
+    p.sdt.dt2 = ff_of(sp->dt * sp->dt);
+    p.sdt.dt_half = ff_of(0.5 * sp->dt);
+    p.sdt.neg_dt = ff_of(-sp->dt);
+    p.dt_range = sp->dt > 0x1p-24 && sp->dt < 0x1p24 ? 1.0f : std::nanf("");
     p.tol_dt = (sp->kepler_tol > 0 ? sp->kepler_tol : KEP_TOL) * sp->dt;
     p.starter = sp->starter;
     p.kill = sp->kill_encounters;

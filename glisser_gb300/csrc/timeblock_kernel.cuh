@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, LEARNED ? GLISSER_TB_MIN_BLOCKS
 {
     extern __shared__ __align__(128) double stage[];
     __shared__ CtaShared sh;
-    load_planet_constants(sh, p.npl, m, rh, pid);
+    load_planet_constants(p, sh, p.npl, m, rh, pid);
     init_barriers(sh);
     __syncthreads();
     uint32_t phase[2] = { 0, 0 };
