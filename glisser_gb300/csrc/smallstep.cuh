@@ -25,15 +25,16 @@
 //            equation itself: fd needs ~2^-46, and this form multiplies the
 //            errors of q2 and q3 by X and tau^2 / 6.
 //
-// Bound: issue (about 1,250 FP32 and integer instructions a step with four
-// planets, ~10 cycles of the 128 lanes; twelve FP64 instructions are 6 cycles of
-// the FP64 pipe).  The line at tau^2 = 1e-3: up to there the error of a drift is that of FP64
-// (position 6e-17 rms of |r| against 6e-17, velocity 5e-17 to 1.4e-16 of |v|
-// against 7e-17 for the coefficients correctly rounded); at 1e-3..2e-3 it is
+// Bound: issue (about 1,400 instructions a step with four planets, 11 cycles of
+// the 128 lanes, at 80 % of the issue slots; twelve FP64 instructions are 6 cycles
+// of the FP64 pipe).  Packed pairs (fma.rn.f32x2) do not help: each takes two
+// issue cycles.  The line at tau^2 = 1e-3: up to there the error of a drift is that
+// of FP64 (position 6e-17 rms of |r| against 6e-17, velocity 5e-17 to 1.4e-16 of
+// |v| against 7e-17 for the coefficients correctly rounded); at 1e-3..2e-3 it is
 // 3.4e-16.  Measured on GB300, before (every drift general) and after: 1e6
-// particles x 1,024 steps with four giants 98.6 -> 48.6 ms; 2e6 planet crossers
-// x 100 steps 16.6 -> 6.0 ms; 2,000 particles x 128 steps 643 -> 358 us;
-// 256 ensembles, 1.5e6 particles x 512 steps, 80 -> 44.6 ms.  Position error of
+// particles x 1,024 steps with four giants 98.6 -> 45.5 ms; 2e6 planet crossers
+// x 100 steps 16.6 -> 5.8 ms; 2,000 particles x 128 steps 643 -> 336 us;
+// 256 ensembles, 1.5e6 particles x 512 steps, 80 -> 37.3 ms.  Position error of
 // those blocks against long double: giants 1.49e-14 -> 1.01e-14 rms, belt
 // 2.34e-14 -> 1.64e-14, crossers 8.6e-16 -> 7.2e-16, scattered disk
 // 3.5e-15 -> 3.0e-15.
@@ -68,18 +69,24 @@ __device__ __forceinline__ ff ff_sqr_u(ff a)
     return { p, __fmaf_rn(__fadd_rn(a.hi, a.hi), a.lo, e) };
 }
 
+__device__ __forceinline__ ff ff_sqr_lo(ff a)       // the same with lo^2
+{
+    const ff s = ff_sqr_u(a);
+    return { s.hi, __fmaf_rn(a.lo, a.lo, s.lo) };
+}
+
 __device__ __forceinline__ ff ff_add_u(ff a, ff b)
 {
     const ff s = ff_two_sum(a.hi, b.hi);
     return { s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)) };
 }
 
-// a . b and |a|^2 of 3-vectors, renormalised
+// a . b and |a|^2 of 3-vectors
 __device__ __forceinline__ ff ff_sum3(ff p, ff q, ff r)
 {
     const ff s = ff_two_sum(p.hi, q.hi);
     const ff t = ff_two_sum(s.hi, r.hi);
-    return ff_fast_two_sum(t.hi, __fadd_rn(__fadd_rn(s.lo, t.lo), __fadd_rn(__fadd_rn(p.lo, q.lo), r.lo)));
+    return { t.hi, __fadd_rn(__fadd_rn(s.lo, t.lo), __fadd_rn(__fadd_rn(p.lo, q.lo), r.lo)) };
 }
 
 __device__ __forceinline__ ff ff_dot3(ff ax, ff ay, ff az, ff bx, ff by, ff bz)
@@ -100,11 +107,15 @@ static __device__ __noinline__ double ff_widen_rare(float hi, float lo) { return
 // 24 significant bits, lo = the (signed) rest rounded to 24: |d - hi - lo| <
 // 2^-49 |d|, for |d| < 2^127.  ff_split counts leading zeros to place lo; here
 // the conversion instruction does.  Zero and |d| < 2^-70 (where lo's unit would
-// leave the float range) take ff_split.
-__device__ __forceinline__ ff ff_split_fast(double d)
+// leave the float range) are rare: they take ff_split.
+__device__ __forceinline__ bool split_is_rare(double d)
+{
+    return ((unsigned)__double2hiint(d) & 0x7fffffffu) < ((1023u - 70u) << 20);
+}
+
+__device__ __forceinline__ ff split_common(double d)
 {
     const unsigned hw = (unsigned)__double2hiint(d), lw = (unsigned)__double2loint(d);
-    if ((hw & 0x7fffffffu) < ((1023u - 70u) << 20)) return ff_split_rare(d);
     // exponent and top 23 significand bits in a float's places; rebiasing from
     // 1023 to 127 adds -896 << 23, 0x40000000 modulo 2^32; bit 28 rounds
     const unsigned f = __funnelshift_l(lw, hw, 3);
@@ -116,21 +127,63 @@ __device__ __forceinline__ ff ff_split_fast(double d)
     return { __uint_as_float(h), __fmul_rn(rest, __uint_as_float(unit)) };
 }
 
+__device__ __forceinline__ ff ff_split_fast(double d)
+{
+    if (split_is_rare(d)) return ff_split_rare(d);
+    return split_common(d);
+}
+
+// Three at once, with one branch for the rare ones.
+__device__ __forceinline__ void ff_split3(double x, double y, double z, ff& fx, ff& fy, ff& fz)
+{
+    fx = split_common(x);
+    fy = split_common(y);
+    fz = split_common(z);
+    if (split_is_rare(x) || split_is_rare(y) || split_is_rare(z)) {
+        fx = ff_split_rare(x);
+        fy = ff_split_rare(y);
+        fz = ff_split_rare(z);
+    }
+}
+
 // hi + lo as a double on the integer and FP32 pipes, to ~2^-47 of it (lo
 // enters in units of 2^-46 of hi's binade), for a renormalised pair: hi widened
 // exactly, lo's multiple of the unit added to the magnitude bits.  hi a power
 // of two (the sum may fall into the binade below, whose unit is another), zero
-// or below 2^-76 takes the FP64 addition.
-__device__ __forceinline__ double ff_widen(ff x)
+// or below 2^-76 is rare: it takes the FP64 addition.
+__device__ __forceinline__ bool widen_is_rare(ff x)
 {
-    const unsigned b = __float_as_uint(x.hi), m = b & 0x7fffffffu;
-    if ((b & 0x007fffffu) == 0u || m < ((127u - 76u) << 23)) return ff_widen_rare(x.hi, x.lo);
+    const unsigned b = __float_as_uint(x.hi);
+    return (b & 0x007fffffu) == 0u || fabsf(x.hi) < 0x1p-76f;
+}
+
+__device__ __forceinline__ double widen_common(ff x)
+{
+    const unsigned b = __float_as_uint(x.hi);
     // 2^(46 - e) with hi's sign, so that the multiple is relative to hi's; the
     // FMA rounds it to an integer in the last places of 1.5 * 2^23
     const float scale = __uint_as_float(((127u + 46u + 127u) << 23) - (b & 0xff800000u));
     const int k = __float_as_int(__fmaf_rn(x.lo, scale, 12582912.0f)) - 0x4b400000;
-    const unsigned hw = (m >> 3) + ((1023u - 127u) << 20) + (b & 0x80000000u);
+    const unsigned hw = ((b & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20) + (b & 0x80000000u);
     return __longlong_as_double((long long)((unsigned long long)hw << 32 | (b << 29)) + ((long long)k << 6));
+}
+
+__device__ __forceinline__ double ff_widen(ff x)
+{
+    if (widen_is_rare(x)) return ff_widen_rare(x.hi, x.lo);
+    return widen_common(x);
+}
+
+__device__ __forceinline__ void ff_widen3(ff x, ff y, ff z, double& dx, double& dy, double& dz)
+{
+    dx = widen_common(x);
+    dy = widen_common(y);
+    dz = widen_common(z);
+    if (widen_is_rare(x) || widen_is_rare(y) || widen_is_rare(z)) {
+        dx = ff_widen_rare(x.hi, x.lo);
+        dy = ff_widen_rare(y.hi, y.lo);
+        dz = ff_widen_rare(z.hi, z.lo);
+    }
 }
 
 // 1/x by the special-function unit (~1 unit in the last place)
@@ -203,9 +256,9 @@ __device__ __forceinline__ bool small_drift(ff rx, ff ry, ff rz, ff vx, ff vy, f
     // below its last place and so never rounded up to it -- a bias of 8e-16 in the
     // Sun's pull, which adds up over the steps
     const ff ri2 = ff_rcp(r2);
-    const ff m2 = ff_mul(muh, ri2);                                   // mu dt^2 / (2 r0^2)
-    const ff th = ff_mul(m2, rinv);                                   // tau^2 / 2
-    const ff b = ff_mul(ff_mul_u(c.dt2, ri2), v2);                    // (v dt / r0)^2
+    const ff m2 = ff_mul_u(muh, ri2);                                 // mu dt^2 / (2 r0^2)
+    const ff th = ff_mul_u(m2, rinv);                                 // tau^2 / 2
+    const ff b = ff_mul_u(ff_mul_u(c.dt2, ri2), v2);                  // (v dt / r0)^2
     const ff X = ff_mul(ff_mul_u(c.dt_half, ri2), u);
     // A = 2 tau^2 - b and 6 Y = tau^2 - A = b - tau^2
     const ff A = ff_add_u(ff_scale(th, 4.0f), ff_neg(b));
@@ -257,7 +310,7 @@ __device__ __forceinline__ bool small_drift(ff rx, ff ry, ff rz, ff vx, ff vy, f
     q3.lo = __fmaf_rn(3.0f * s2, dw, q3.lo);
 
     const ff o2 = ff_fast_two_sum(1.0f, q2.hi), o3 = ff_fast_two_sum(1.0f, q3.hi);
-    d.h = ff_mul(m2, ff{ o2.hi, o2.lo + q2.lo });
+    d.h = ff_mul_u(m2, ff{ o2.hi, o2.lo + q2.lo });
     d.f1 = ff_neg(ff_mul_u(d.h, rinv));
     const ff p = ff_mul(ff_mul_u(th, ff_third()), ff{ o3.hi, o3.lo + q3.lo });
     d.gdt = ff_mul_u(c.neg_dt, p);

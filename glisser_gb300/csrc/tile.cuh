@@ -162,18 +162,21 @@ constexpr float KICK_MDT_MIN = 0x1p-40f, KICK_MDT_MAX = 0x1p30f;
 __device__ __forceinline__ void planet_kick(const ff* L, int j, ff rx, ff ry, ff rz, ff& sx, ff& sy, ff& sz,
                                             uint16_t& flags, uint32_t& border, const CtaShared& sh)
 {
-    const ff dx = ff_add(rx, ff_neg(L[3 * j]));
-    const ff dy = ff_add(ry, ff_neg(L[3 * j + 1]));
-    const ff dz = ff_add(rz, ff_neg(L[3 * j + 2]));
-    const ff rad = ff_sqr3(dx, dy, dz);
+    // differences not renormalised: near the planet their lo may reach far above
+    // hi's last place, so the squares keep lo^2
+    const ff dx = ff_add_u(rx, ff_neg(L[3 * j]));
+    const ff dy = ff_add_u(ry, ff_neg(L[3 * j + 1]));
+    const ff dz = ff_add_u(rz, ff_neg(L[3 * j + 2]));
+    const ff rad = ff_norm(ff_sum3(ff_sqr_lo(dx), ff_sqr_lo(dy), ff_sqr_lo(dz)));
     const PlanetConst& q = sh.pk[j];
     ff fac;
     if (rad.hi > q.near2 && rad.hi < KICK_R2_MAX) {
         // m |dr|^-3 from the seed y: m y^3 (1 + 1.5 e + 1.875 e^2), e = 1 - |dr|^2 y^2
         const float y = rsqrtf(rad.hi);
         const float e = rsqrt_residual(rad, y);
-        const ff my3 = ff_mul_u(q.mdt, ff_mul_f(ff_two_prod(y, y), y));
-        fac = ff_fast_two_sum(my3.hi, __fmaf_rn(my3.hi, __fmul_rn(e, __fmaf_rn(1.875f, e, 1.5f)), my3.lo));
+        const ff y2 = ff_two_prod(y, y), y3 = ff_two_prod(y2.hi, y);
+        const ff my3 = ff_mul_u(q.mdt, ff{ y3.hi, __fmaf_rn(y2.lo, y, y3.lo) });
+        fac = { my3.hi, __fmaf_rn(my3.hi, __fmul_rn(e, __fmaf_rn(1.875f, e, 1.5f)), my3.lo) };
     } else {
         if (flags == 0) {
             // rad.hi - rh2.hi is exact near the threshold (Sterbenz), so the FP32
@@ -273,9 +276,7 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
             vy[k] = fma(a0y, hdt, vy[k]);
             vz[k] = fma(a0z, hdt, vz[k]);
         }
-        fx[k] = ff_split_fast(rx[k]);
-        fy[k] = ff_split_fast(ry[k]);
-        fz[k] = ff_split_fast(rz[k]);
+        ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
         f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
         fri[k] = ff_rsqrt(f2[k]);
         if (!(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX)) fri[k].hi = __int_as_float(0x7fc00000);
@@ -331,9 +332,7 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                 const float q3 = sh.muh.hi * fri[k].hi * (fri[k].hi * fri[k].hi);
                 bool small = p.starter != STARTER_CLASSIC && q3 < 0.5f * SMALL_DRIFT_TAU2;
                 if (small) {
-                    wx = ff_split_fast(vx[k]);
-                    wy = ff_split_fast(vy[k]);
-                    wz = ff_split_fast(vz[k]);
+                    ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
                     small = small_drift(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
                 }
                 if (small) {
@@ -342,20 +341,20 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                     const ff cx = ff_norm(ff_add_u(ff_mul_u(sd.f1, fx[k]), ff_mul_u(sd.gdt, wx)));
                     const ff cy = ff_norm(ff_add_u(ff_mul_u(sd.f1, fy[k]), ff_mul_u(sd.gdt, wy)));
                     const ff cz = ff_norm(ff_add_u(ff_mul_u(sd.f1, fz[k]), ff_mul_u(sd.gdt, wz)));
-                    rx[k] += fma(p.dt, vx[k], ff_widen(cx));
-                    ry[k] += fma(p.dt, vy[k], ff_widen(cy));
-                    rz[k] += fma(p.dt, vz[k], ff_widen(cz));
+                    double dx, dy, dz;
+                    ff_widen3(cx, cy, cz, dx, dy, dz);
+                    rx[k] += fma(p.dt, vx[k], dx);
+                    ry[k] += fma(p.dt, vy[k], dy);
+                    rz[k] += fma(p.dt, vz[k], dz);
                     const ff ox = fx[k], oy = fy[k], oz = fz[k];
-                    fx[k] = ff_split_fast(rx[k]);
-                    fy[k] = ff_split_fast(ry[k]);
-                    fz[k] = ff_split_fast(rz[k]);
+                    ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
                     // |r'|^2 in FP64 (three instructions of a pipe with room), then
                     // 1/|r'| in float-float
                     f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
                     fri[k] = ff_rsqrt(f2[k]);
                     // v' = v + (fd r + (gd - 1) v)
                     const ff gd1 = ff_neg(ff_mul_u(sd.h, fri[k]));
-                    const ff fd = ff_mul(sd.fdr, fri[k]);
+                    const ff fd = ff_mul_u(sd.fdr, fri[k]);
                     gx = ff_add_u(ff_mul_u(fd, ox), ff_mul_u(gd1, wx));
                     gy = ff_add_u(ff_mul_u(fd, oy), ff_mul_u(gd1, wy));
                     gz = ff_add_u(ff_mul_u(fd, oz), ff_mul_u(gd1, wz));
@@ -376,9 +375,7 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                     evals += d.evals;
                     if constexpr (LEARNED) nets += d.net;
                     wide += d.wide;
-                    fx[k] = ff_split_fast(rx[k]);
-                    fy[k] = ff_split_fast(ry[k]);
-                    fz[k] = ff_split_fast(rz[k]);
+                    ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
                     f2[k] = ff_split_fast(r2[k]);
                     fri[k] = ff_split_fast(rinv[k]);
                 }
@@ -395,13 +392,12 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                             planet_kick64(Ld, j, rx[k], ry[k], rz[k], aax, aay, aaz, fl, border, sh);
                     }
                 } else {
-                    // dt (h0 - sum of the planets' pulls).  The planet loop stays rolled: the kernel is bound by
-                    // instruction fetch, and the unrolled four-planet
-                    // float-float kick measured 9-12 % slower (the ensemble
-                    // kernel and the single-system plain-giants kernel)
+                    // dt (h0 - sum of the planets' pulls)
                     sx = L[0]; sy = L[1]; sz = L[2];
                     if constexpr (NP > 0) {
-#pragma unroll 1
+                        // unrolled up to four planets: 2 % faster than rolled on the
+                        // giants (47.5 against 48.5 ms) since the kernel is bound by issue
+#pragma unroll (NP <= 4 ? NP : 1)
                         for (int j = 1; j <= NP; j++) planet_kick(L, j, fx[k], fy[k], fz[k], sx, sy, sz, fl, border, sh);
                     } else {
                         for (int j = 1; j <= np; j++) planet_kick(L, j, fx[k], fy[k], fz[k], sx, sy, sz, fl, border, sh);
@@ -433,13 +429,18 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                 }
                 if constexpr (KICK64) {
                     const double kc = last ? hdt : p.dt;
-                    vx[k] += fma(aax, kc, ff_widen(ff_norm(gx)));
-                    vy[k] += fma(aay, kc, ff_widen(ff_norm(gy)));
-                    vz[k] += fma(aaz, kc, ff_widen(ff_norm(gz)));
+                    double dx, dy, dz;
+                    ff_widen3(ff_norm(gx), ff_norm(gy), ff_norm(gz), dx, dy, dz);
+                    vx[k] += fma(aax, kc, dx);
+                    vy[k] += fma(aay, kc, dy);
+                    vz[k] += fma(aaz, kc, dz);
                 } else {
-                    vx[k] += ff_widen(ff_norm(ff_add_u(gx, sx)));
-                    vy[k] += ff_widen(ff_norm(ff_add_u(gy, sy)));
-                    vz[k] += ff_widen(ff_norm(ff_add_u(gz, sz)));
+                    double dx, dy, dz;
+                    ff_widen3(ff_norm(ff_add_u(gx, sx)), ff_norm(ff_add_u(gy, sy)), ff_norm(ff_add_u(gz, sz)), dx, dy,
+                              dz);
+                    vx[k] += dx;
+                    vy[k] += dy;
+                    vz[k] += dz;
                 }
             }
         }

@@ -43,7 +43,7 @@ void drift(int n, double dt, double mu, double* rv, int* ok)
         for (int k = 0; k < 3; k++)
             r[k] += std::fma(dt, v[k], ff_widen(ff_norm(ff_add_u(ff_mul_u(d.f1, f[k]), ff_mul_u(d.gdt, w[k])))));
         const ff n2 = ff_split_fast(std::fma(r[0], r[0], std::fma(r[1], r[1], r[2] * r[2])));
-        const ff ri = ff_rsqrt(n2), gd1 = ff_neg(ff_mul_u(d.h, ri)), fd = ff_mul(d.fdr, ri);
+        const ff ri = ff_rsqrt(n2), gd1 = ff_neg(ff_mul_u(d.h, ri)), fd = ff_mul_u(d.fdr, ri);
         for (int k = 0; k < 3; k++) v[k] += ff_widen(ff_norm(ff_add_u(ff_mul_u(fd, f[k]), ff_mul_u(gd1, w[k]))));
     }
 }
