@@ -1,5 +1,5 @@
-// FP64 reciprocal square root and reciprocal seeded by the FP32 special-
-// function unit.
+// FP64 reciprocal square root and quotient seeded by the FP32 special-function
+// unit.
 //
 // On GB300 every FP64 instruction is scarce (the FP64 pipe issues at 1/64 of
 // the FP32 rate), so the seed is built without FP64 instructions at all: the
@@ -8,7 +8,6 @@
 // are moved back into a double the same way.  One third-order correction
 // (Householder) then brings the ~2^-22 seed to full double precision:
 //   rsqrt: e = 1 - x y^2,  y' = y (1 + e/2 + 3e^2/8)      (5 FP64 ops)
-//   rcp:   e = 1 - x y,    y' = y (1 + e + e^2)           (3 FP64 ops)
 // the residual error is O(e^3) ~ 1e-20, below double rounding.  Arguments
 // outside the normal float range (and NaN/inf) take the library routines.
 // The drift's own 1/|r| (rsqrt_lean, below the float-float arithmetic) keeps
@@ -52,13 +51,16 @@ __device__ __forceinline__ double rsqrt_fast(double x)
     return fma(y * e, p, y);
 }
 
-__device__ __forceinline__ double rcp_fast(double x)
+// a / b to ~2^-45 from the FP32 reciprocal of b (seed 2^-22.4) and one
+// correction with the remainder, for the Newton correction h = f / f' of a pass
+// that is judged, or small next to s: 3 FP64 ops.
+__device__ __forceinline__ double quotient_fast(double a, double b)
 {
-    int hi = __double2hiint(x);
-    if (!float_range(hi)) return 1.0 / x;
-    double y = widen_bits(__frcp_rn(seed_float(hi)));
-    double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
+    int hi = __double2hiint(b);
+    if (!float_range(hi)) return a / b;
+    const double y = widen_bits(__frcp_rn(seed_float(hi)));
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
 }
 
 // m x^(-3/2) from m15 = 1.5 m, for a planet's pull m dr / |dr|^3 (x = |dr|^2):

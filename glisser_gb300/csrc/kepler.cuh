@@ -10,7 +10,7 @@
 // FP64 at a small fraction of its FP32 rate, so the solver is written to
 // minimise FP64 instructions, moving to the FP32 and integer pipes what
 // provably does not need FP64:
-//  * one FP64 reciprocal per Newton pass: the quartic correction is the
+//  * one FP64 quotient per Newton pass: the quartic correction is the
 //    series reversion  ds = -h - A h^2 + (B - 2A^2) h^3  (h = f/f',
 //    A = f''/2f', B = f'''/6f'), which has the same fourth-order
 //    convergence as the reference's three nested divisions; only h is
@@ -36,9 +36,10 @@
 //  * the accepted correction's fold and the float-float sums return to FP64
 //    by integer additions to the bit patterns (f64_add_tiny, ff_to_f64 in
 //    fastmath.cuh);
-//  * the Stumpff series is evaluated by Horner in x = alpha s^2; arguments
-//    with |x| >= 0.1 are quartered and rebuilt with the double-angle
-//    identities (c0,c1,c2,c3 as in Danby eq. 6.9.15).  For a small step
+//  * the Stumpff series is evaluated by Horner in x = alpha s^2, of a length by
+//    |x| (to x^3, x^6 or x^11); arguments with |x| >= 4.5 are quartered and
+//    rebuilt with the double-angle identities (c0,c1,c2,c3 as in Danby eq.
+//    6.9.15).  For a small step
 //    (|x| < 2e-3, tau^2 < 2e-3) the corrections to G2 = s^2/2 and all of G3
 //    need far fewer than 53 bits and are formed in float-float: three FP64
 //    instructions instead of twelve;
@@ -105,6 +106,36 @@ __device__ __forceinline__ void stumpff_short(double x, double& c2, double& c3)
 // The time-block kernels are bound by the FP64 pipe, so here and in the
 // solver below float-to-double sums and the residual-accepted fold go through
 // the integer pipe (ff_to_f64, f64_add_tiny).
+// c2, c3 to x^11: enough when |x| < 4.5 (the x^12 terms are below 2e-19), steps
+// up to two radians of eccentric anomaly.  22 FP64 instructions where quartering
+// the argument and rebuilding by the double-angle identities took 12 and about
+// nine for each quartering (two or three of them, and a bit of accuracy each).
+__device__ __forceinline__ void stumpff_wide(double x, double& c2, double& c3)
+{
+    c2 = fma(x, -1.0 / 620448401733239439360000.0, 1.0 / 1124000727777607680000.0);
+    c2 = fma(x, c2, -1.0 / 2432902008176640000.0);
+    c2 = fma(x, c2, 1.0 / 6402373705728000.0);
+    c2 = fma(x, c2, -1.0 / 20922789888000.0);
+    c2 = fma(x, c2, 1.0 / 87178291200.0);
+    c2 = fma(x, c2, -1.0 / 479001600.0);
+    c2 = fma(x, c2, 1.0 / 3628800.0);
+    c2 = fma(x, c2, -1.0 / 40320.0);
+    c2 = fma(x, c2, 1.0 / 720.0);
+    c2 = fma(x, c2, -1.0 / 24.0);
+    c2 = fma(x, c2, 0.5);
+    c3 = fma(x, -1.0 / 15511210043330985984000000.0, 1.0 / 25852016738884976640000.0);
+    c3 = fma(x, c3, -1.0 / 51090942171709440000.0);
+    c3 = fma(x, c3, 1.0 / 121645100408832000.0);
+    c3 = fma(x, c3, -1.0 / 355687428096000.0);
+    c3 = fma(x, c3, 1.0 / 1307674368000.0);
+    c3 = fma(x, c3, -1.0 / 6227020800.0);
+    c3 = fma(x, c3, 1.0 / 39916800.0);
+    c3 = fma(x, c3, -1.0 / 362880.0);
+    c3 = fma(x, c3, 1.0 / 5040.0);
+    c3 = fma(x, c3, -1.0 / 120.0);
+    c3 = fma(x, c3, 1.0 / 6.0);
+}
+
 __device__ __forceinline__ GFun gfuns(double s, double alpha, bool small_step)
 {
     const double s2 = s * s;
@@ -145,8 +176,10 @@ __device__ __forceinline__ GFun gfuns(double s, double alpha, bool small_step)
         // warp-uniform: every lane in this pass has a small argument (and
         // some lane a step too large for the float-float tier)
         stumpff_short(x, c2, c3);
-    } else if (fabs(x) < 0.1) {
+    } else if (lt_nonneg(ax, 0.1)) {
         stumpff_small(x, c2, c3);
+    } else if (lt_nonneg(ax, 4.5)) {
+        stumpff_wide(x, c2, c3);
     } else {
         // quarter the argument until |x| < 0.1, then rebuild (bounded: x
         // finite needs at most ~520 quarterings; non-finite x stops at 600)
@@ -505,7 +538,8 @@ __device__ __forceinline__ void fold_small(GFun& g, double& ds, double f, double
 //     accepted solution carries an O(tol^2) error instead of O(tol);
 //   - predicted acceptance (newton_terms): ds is the whole reverted
 //     correction, folded by Taylor expansion through ds^3 (G0' = -alpha G1,
-//     G1' = G0, G2' = G1, G3' = G2):
+//     G1' = G0, G2' = G1, G3' = G2; the ds^3 terms only where |ds| is 2^-18 of
+//     s or more):
 //       G3 + ds (G2 + ds/2 (G1 + ds/3 G0)),
 //       G2 + ds (G1 + ds/2 (G0 - alpha ds/3 G1)),
 //       G1 + ds (G0 - alpha ds/2 (G1 + ds/3 G0));
@@ -523,16 +557,22 @@ __device__ __forceinline__ bool kepler_newton(double& s, double dt, double r0, d
         }
         const double g0 = gfun_g0(g, alpha);
         const double fp = fma(r0, g0, fma(u, g.g1, mu * g.g2));
-        const double h = f * rcp_fast(fp);
+        const double h = quotient_fast(f, fp);
         float x_step, x_root;
         const int pass = newton_terms(f, fp, h, r0, u, mu, alpha, g0, g, tol, x_step, x_root);
         if (pass == NEWTON_WILD) return false;
         if (pass == NEWTON_PREDICTED) {
             ds = fma(-h, f64_of_f32(x_root), -h);
-            const double t = ds * (1.0 / 3.0), hd = 0.5 * ds;
-            const double q1 = fma(t, g0, g.g1);
+            const double hd = f64_half(ds);
+            double q1 = g.g1, q0 = g0;
+            if (!(fabsf(f32_trunc(ds)) < 0x1p-18f * fabsf(f32_trunc(s)))) {
+                // the ds^3 terms, above 2^-54 of G only for a larger correction
+                const double t = ds * (1.0 / 3.0);
+                q1 = fma(t, g0, g.g1);
+                q0 = fma(-alpha * t, g.g1, g0);
+            }
             const double n3 = fma(ds, fma(hd, q1, g.g2), g.g3);
-            const double n2 = fma(ds, fma(hd, fma(-alpha * t, g.g1, g0), g.g1), g.g2);
+            const double n2 = fma(ds, fma(hd, q0, g.g1), g.g2);
             const double n1 = fma(ds, fma(-alpha * hd, q1, g0), g.g1);
             g.g3 = n3;
             g.g2 = n2;

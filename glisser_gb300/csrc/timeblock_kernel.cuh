@@ -9,30 +9,26 @@ namespace {
 
 using namespace tile;
 
-// CTAs per SM the register allocation is sized for.  Once the drift's
-// reciprocal square root and small-step Stumpff tier moved most of their
-// FP64 work to the FP32 and integer pipes, the kernel became latency-bound
-// with neither pipe saturated, and resident warps count: 16 CTAs of 64
-// threads (64 registers, a few dozen bytes of spills; 32-step planet-log
-// chunks, so that shared memory admits 16 with four planets) measured 7 %
-// faster than 10 CTAs at 80 registers on the plain-giants workload and 2.5 %
-// on the scattered disk; 18 and 20 CTAs spill more.
+// CTAs per SM the register allocation is sized for: 16 CTAs of 64 threads (64
+// registers, a few dozen bytes of spills; 32-step planet-log chunks, so that
+// shared memory admits 16 with four planets).  12 CTAs measured 3 % slower on
+// the giants and 5 % on planet crossers, 8 CTAs 4 and 9 %; only a run that leaves
+// the SMs nearly empty (2,000 particles) gains, 4 to 6 %.
 #ifndef GLISSER_TB_MIN_BLOCKS
 #define GLISSER_TB_MIN_BLOCKS 16
 #endif
 
 // The learned-starter kernel runs the network per lane, inline, only where
-// the series starter is outside its domain.  Its register allocation follows
-// the plain kernel's occupancy (16 CTAs of 64 per SM: 64 registers), so that
-// the network costs no occupancy on the steps that do not run it: at 80
-// registers (12 CTAs) it ran 0.991x the plain kernel on the scattered disk,
-// where 0.1 % of drifts take the network, and 1.062x on the close-eccentric
-// workload, where every drift does; at 64 registers 1.016x and 1.071x (the
-// spills sit around the network).  The network's shape
-// (mlp_forward: four rows of the hidden layer per pass, two activation
-// reads in flight) was chosen for a register budget.
+// the series starter is outside its domain.  Sized for 14 CTAs of 64 (72
+// registers): the network's registers cost less there than its spills at 16
+// (64 registers), 3.41 against 4.43 ms for a 128-step block of 100,000
+// close-eccentric particles, 14.55 against 14.62 ms for 64 steps of 1e6, and
+// 5.93 against 5.78 ms on 1e6 scattered-disk particles, where 0.1 % of drifts
+// take the network.  The network's shape (mlp_forward: four rows of the hidden
+// layer per pass, two activation reads in flight) was chosen for a register
+// budget.
 #ifndef GLISSER_TB_MIN_BLOCKS_LEARNED
-#define GLISSER_TB_MIN_BLOCKS_LEARNED 16
+#define GLISSER_TB_MIN_BLOCKS_LEARNED 14
 #endif
 constexpr int TB_NET_ROWS = 4;
 constexpr int TB_NET_QU = 2;
