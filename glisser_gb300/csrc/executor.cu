@@ -718,7 +718,7 @@ bool Executor::step_block(double* cpu_ms, double* gpu_ms)
         int nxt = d.cur ^ 1;
         int rc = launch_partition(&d.buf[d.cur].p, &d.buf[nxt].p, n_range, d.d_scratch, d.d_ctr + 2, d.d_ctr + 3,
                                   d.main);
-        launches_total_ += 3;   // count, scan, scatter
+        launches_total_ += 2;   // count, scatter
         if (rc != GLISSER_OK) throw CudaError("partition launch failed");
         ck(cudaMemcpyAsync(d.h_ctr, d.d_ctr, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, d.main), "counters");
         ck(cudaMemcpyAsync(d.h_evals, d.d_evals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, d.main),

@@ -4,11 +4,18 @@
 // executor (src/executor.cu:663-665, 784-790, 865-869) with a deterministic
 // order, so the host mirror and every output file are reproducible.
 //
-// Three launches over tiles of TILE particles: per-tile category counts by
-// warp ballot, one exclusive scan of the tile counts, and a scatter in which
-// each tile recomputes its ranks and writes the 12 particle arrays to the
-// output buffer.  HBM traffic is one read of the flags plus one read and one
-// write of the 96-byte particle record.
+// Two launches over at most RANGES contiguous ranges of particles, one CTA each:
+// the counts of each range's categories, then a scatter in which every CTA adds
+// up the counts before its own (a few KB from L2) and walks its range in tiles of
+// TILE, writing the 12 particle arrays to the output buffer.  HBM traffic is one
+// read of the flags plus one read and one write of the 90-byte particle record.
+//
+// Bound: HBM.  A tile's record is read before its flags are ranked, and the next
+// tile's before this one's is written, so that loads are in flight across the
+// barriers.  A separate scan launch of one CTA between the two (per-tile
+// counts, one particle per thread, the record read after the ranks) took 55 us
+// for 1e6 particles and 197 us for 4e6; this takes 35 and 119 us, 0.76 and 0.89
+// of the measured copy rate, and 8.4 against 14.5 us for 5,000.
 #include <cuda.h>
 
 #include <cstdio>
@@ -21,7 +28,9 @@ namespace glisser {
 namespace {
 
 constexpr int TILE = 256;
-constexpr int SCAN_THREADS = 1024;
+// three CTAs of 256 threads (80 registers: two records) on each of GB300's 152 SMs; four at
+// 64 registers measured 38 against 35 us for 1e6 particles
+constexpr uint32_t RANGES = 152 * 3;
 
 __device__ __forceinline__ int category(uint16_t f)
 {
@@ -30,100 +39,121 @@ __device__ __forceinline__ int category(uint16_t f)
     return 2;
 }
 
-// Per-tile counts of categories 0 and 1 into counts[2*tile + {0,1}].
-__global__ void __launch_bounds__(TILE) count_kernel(const uint16_t* __restrict__ flags, uint32_t n, uint32_t* counts)
+// Sums of two values over the CTA, returned to every thread.
+__device__ __forceinline__ void cta_sum2(uint32_t& a, uint32_t& b, uint32_t (*buf)[TILE / 32])
 {
-    __shared__ uint32_t warp_c[2][TILE / 32];
-    uint32_t i = blockIdx.x * TILE + threadIdx.x;
-    int cat = i < n ? category(flags[i]) : 2;
-    unsigned b0 = __ballot_sync(0xffffffffu, cat == 0);
-    unsigned b1 = __ballot_sync(0xffffffffu, cat == 1);
+    a = __reduce_add_sync(0xffffffffu, a);
+    b = __reduce_add_sync(0xffffffffu, b);
     if ((threadIdx.x & 31) == 0) {
-        warp_c[0][threadIdx.x >> 5] = __popc(b0);
-        warp_c[1][threadIdx.x >> 5] = __popc(b1);
+        buf[0][threadIdx.x >> 5] = a;
+        buf[1][threadIdx.x >> 5] = b;
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
-        uint32_t s = 0;
-        for (int w = 0; w < TILE / 32; w++) s += warp_c[threadIdx.x][w];
-        counts[2 * blockIdx.x + threadIdx.x] = s;
+    a = b = 0;
+#pragma unroll
+    for (int w = 0; w < TILE / 32; w++) {
+        a += buf[0][w];
+        b += buf[1][w];
+    }
+    __syncthreads();
+}
+
+// Counts of categories 0 and 1 of range b = [b * per, (b + 1) * per) into
+// counts[2 * b + {0, 1}].
+__global__ void __launch_bounds__(TILE) count_kernel(const uint16_t* __restrict__ flags, uint32_t n, uint32_t per,
+                                                     uint32_t* counts)
+{
+    __shared__ uint32_t buf[2][TILE / 32];
+    const uint32_t lo = blockIdx.x * per, hi = n - lo < per ? n : lo + per;
+    uint32_t c0 = 0, c1 = 0;
+#pragma unroll 4
+    for (uint32_t i = lo + threadIdx.x; i < hi; i += TILE) {
+        const int cat = category(flags[i]);
+        c0 += cat == 0;
+        c1 += cat == 1;
+    }
+    cta_sum2(c0, c1, buf);
+    if (threadIdx.x == 0) {
+        counts[2 * blockIdx.x] = c0;
+        counts[2 * blockIdx.x + 1] = c1;
     }
 }
 
-// Exclusive scan of the per-tile counts in place (single CTA), totals out.
-__global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(uint32_t* counts, uint32_t ntiles, uint32_t* n0, uint32_t* n1)
+struct Record {
+    double f[9];
+    uint32_t dti, id;
+    uint16_t flags;
+};
+
+__device__ __forceinline__ Record read_record(const glisser_particles& p, uint32_t i, bool valid)
 {
-    __shared__ uint32_t part[2][SCAN_THREADS];
-    uint32_t per = (ntiles + SCAN_THREADS - 1) / SCAN_THREADS;
-    uint32_t lo = threadIdx.x * per;
-    uint32_t hi = min(lo + per, ntiles);
-    uint32_t s0 = 0, s1 = 0;
-    for (uint32_t t = lo; t < hi; t++) {
-        s0 += counts[2 * t];
-        s1 += counts[2 * t + 1];
+    Record r = {};
+    if (valid) {
+        r.flags = p.flags[i];
+        r.f[0] = p.rx[i]; r.f[1] = p.ry[i]; r.f[2] = p.rz[i];
+        r.f[3] = p.vx[i]; r.f[4] = p.vy[i]; r.f[5] = p.vz[i];
+        r.f[6] = p.ax[i]; r.f[7] = p.ay[i]; r.f[8] = p.az[i];
+        r.dti = p.deathtime_index[i];
+        r.id = p.id[i];
     }
-    part[0][threadIdx.x] = s0;
-    part[1][threadIdx.x] = s1;
-    __syncthreads();
-    // Hillis-Steele inclusive scan over the 1024 partial sums
-    for (int off = 1; off < SCAN_THREADS; off <<= 1) {
-        uint32_t a0 = threadIdx.x >= (unsigned)off ? part[0][threadIdx.x - off] : 0;
-        uint32_t a1 = threadIdx.x >= (unsigned)off ? part[1][threadIdx.x - off] : 0;
-        __syncthreads();
-        part[0][threadIdx.x] += a0;
-        part[1][threadIdx.x] += a1;
-        __syncthreads();
-    }
-    uint32_t b0 = part[0][threadIdx.x] - s0;
-    uint32_t b1 = part[1][threadIdx.x] - s1;
-    for (uint32_t t = lo; t < hi; t++) {
-        uint32_t c0 = counts[2 * t], c1 = counts[2 * t + 1];
-        counts[2 * t] = b0;
-        counts[2 * t + 1] = b1;
-        b0 += c0;
-        b1 += c1;
-    }
-    if (threadIdx.x == SCAN_THREADS - 1) {
-        *n0 = part[0][SCAN_THREADS - 1];
-        *n1 = part[1][SCAN_THREADS - 1];
-    }
+    return r;
 }
 
-__global__ void __launch_bounds__(TILE) scatter_kernel(glisser_particles in, glisser_particles out, uint32_t n,
-                                                       const uint32_t* offsets, const uint32_t* n0p,
-                                                       const uint32_t* n1p)
+__global__ void __launch_bounds__(TILE, 3) scatter_kernel(glisser_particles in, glisser_particles out, uint32_t n,
+                                                       uint32_t per, const uint32_t* __restrict__ counts,
+                                                       uint32_t* n0p, uint32_t* n1p)
 {
-    __shared__ uint32_t warp_c[2][TILE / 32];
-    uint32_t i = blockIdx.x * TILE + threadIdx.x;
-    int cat = i < n ? category(in.flags[i]) : 3;
-    unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned b0 = __ballot_sync(0xffffffffu, cat == 0);
-    unsigned b1 = __ballot_sync(0xffffffffu, cat == 1);
-    if (lane == 0) {
-        warp_c[0][warp] = __popc(b0);
-        warp_c[1][warp] = __popc(b1);
+    __shared__ uint32_t buf[2][TILE / 32];
+    __shared__ uint32_t warp_c[2][2][TILE / 32];
+    const uint32_t lo = blockIdx.x * per, hi = n - lo < per ? n : lo + per;
+    Record cur = read_record(in, lo + threadIdx.x, lo + threadIdx.x < hi);
+    // category counts before this range, and in all
+    uint32_t before0 = 0, before1 = 0, all0 = 0, all1 = 0;
+    for (uint32_t b = threadIdx.x; b < gridDim.x; b += TILE) {
+        const uint32_t c0 = counts[2 * b], c1 = counts[2 * b + 1];
+        all0 += c0;
+        all1 += c1;
+        before0 += b < blockIdx.x ? c0 : 0u;
+        before1 += b < blockIdx.x ? c1 : 0u;
     }
-    __syncthreads();
-    if (i >= n) return;
-    uint32_t before0 = 0, before1 = 0;
-    for (unsigned w = 0; w < warp; w++) {
-        before0 += warp_c[0][w];
-        before1 += warp_c[1][w];
+    cta_sum2(before0, before1, buf);
+    cta_sum2(all0, all1, buf);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *n0p = all0;
+        *n1p = all1;
     }
-    unsigned lt = (1u << lane) - 1u;
-    uint32_t r0 = offsets[2 * blockIdx.x] + before0 + __popc(b0 & lt);
-    uint32_t r1 = offsets[2 * blockIdx.x + 1] + before1 + __popc(b1 & lt);
-    uint32_t n0 = *n0p, n1 = *n1p;
-    uint32_t dst;
-    if (cat == 0) dst = r0;
-    else if (cat == 1) dst = n0 + r1;
-    else dst = n0 + n1 + (i - r0 - r1);
-    out.rx[dst] = in.rx[i]; out.ry[dst] = in.ry[i]; out.rz[dst] = in.rz[i];
-    out.vx[dst] = in.vx[i]; out.vy[dst] = in.vy[i]; out.vz[dst] = in.vz[i];
-    out.ax[dst] = in.ax[i]; out.ay[dst] = in.ay[i]; out.az[dst] = in.az[i];
-    out.flags[dst] = in.flags[i];
-    out.deathtime_index[dst] = in.deathtime_index[i];
-    out.id[dst] = in.id[i];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t parity = 0;
+    for (uint32_t base = lo; base < hi; base += TILE, parity ^= 1u) {
+        const uint32_t i = base + threadIdx.x;
+        const Record next = read_record(in, i + TILE, i + TILE < hi);
+        const int cat = i < hi ? category(cur.flags) : 3;
+        const unsigned b0 = __ballot_sync(0xffffffffu, cat == 0), b1 = __ballot_sync(0xffffffffu, cat == 1);
+        if (lane == 0) {
+            warp_c[parity][0][warp] = __popc(b0);
+            warp_c[parity][1][warp] = __popc(b1);
+        }
+        __syncthreads();     // the other parity's counts are rewritten only after the next one
+        uint32_t r0 = before0 + __popc(b0 & lt), r1 = before1 + __popc(b1 & lt);
+#pragma unroll
+        for (unsigned w = 0; w < TILE / 32; w++) {
+            const uint32_t c0 = warp_c[parity][0][w], c1 = warp_c[parity][1][w];
+            r0 += w < warp ? c0 : 0u;
+            r1 += w < warp ? c1 : 0u;
+            before0 += c0;
+            before1 += c1;
+        }
+        if (i < hi) {
+            const uint32_t dst = cat == 0 ? r0 : cat == 1 ? all0 + r1 : all0 + all1 + (i - r0 - r1);
+            out.rx[dst] = cur.f[0]; out.ry[dst] = cur.f[1]; out.rz[dst] = cur.f[2];
+            out.vx[dst] = cur.f[3]; out.vy[dst] = cur.f[4]; out.vz[dst] = cur.f[5];
+            out.ax[dst] = cur.f[6]; out.ay[dst] = cur.f[7]; out.az[dst] = cur.f[8];
+            out.flags[dst] = cur.flags;
+            out.deathtime_index[dst] = cur.dti;
+            out.id[dst] = cur.id;
+        }
+        cur = next;
+    }
 }
 
 __global__ void copy_range_kernel(glisser_particles src, glisser_particles dst, uint32_t begin, uint32_t end)
@@ -156,6 +186,23 @@ size_t partition_scratch_bytes(size_t n)
     return 2 * tiles * sizeof(uint32_t) + 64;
 }
 
+namespace {
+
+// Both launches; counts holds two words per range (at most RANGES ranges, and
+// never more than one per TILE particles).
+int launch_two(const glisser_particles* in, const glisser_particles* out, uint32_t n, uint32_t* counts, uint32_t* n0,
+               uint32_t* n1, cudaStream_t stream)
+{
+    const uint32_t tiles = (uint32_t)(((uint64_t)n + TILE - 1) / TILE);
+    const uint32_t per = (tiles + RANGES - 1) / RANGES * TILE;       // whole tiles per range
+    const uint32_t ranges = (uint32_t)(((uint64_t)n + per - 1) / per);
+    count_kernel<<<ranges, TILE, 0, stream>>>(in->flags, n, per, counts);
+    scatter_kernel<<<ranges, TILE, 0, stream>>>(*in, *out, n, per, counts, n0, n1);
+    return cudaGetLastError() == cudaSuccess ? GLISSER_OK : GLISSER_E_CUDA;
+}
+
+}  // namespace
+
 int launch_partition(const glisser_particles* in, const glisser_particles* out, size_t n, void* scratch,
                      uint32_t* n0, uint32_t* n1, cudaStream_t stream)
 {
@@ -166,12 +213,7 @@ int launch_partition(const glisser_particles* in, const glisser_particles* out, 
         cudaMemsetAsync(n1, 0, sizeof(uint32_t), stream);
         return cudaGetLastError() == cudaSuccess ? GLISSER_OK : GLISSER_E_CUDA;
     }
-    uint32_t tiles = (uint32_t)((n + TILE - 1) / TILE);
-    uint32_t* counts = reinterpret_cast<uint32_t*>(scratch);
-    count_kernel<<<tiles, TILE, 0, stream>>>(in->flags, (uint32_t)n, counts);
-    scan_kernel<<<1, SCAN_THREADS, 0, stream>>>(counts, tiles, n0, n1);
-    scatter_kernel<<<tiles, TILE, 0, stream>>>(*in, *out, (uint32_t)n, counts, n0, n1);
-    return cudaGetLastError() == cudaSuccess ? GLISSER_OK : GLISSER_E_CUDA;
+    return launch_two(in, out, (uint32_t)n, reinterpret_cast<uint32_t*>(scratch), n0, n1, stream);
 }
 
 
@@ -186,11 +228,11 @@ int launch_partition(const glisser_particles* in, const glisser_particles* out, 
 // that glisser_partition keeps in caller-provided scratch live here in a
 // file-scope device array instead.
 //
-// NOALLOC_MAX_PARTICLES bounds n: 2 counts per 256-particle tile, 256 KiB in
-// all, resident on every GPU that loads the library until the process exits.
+// NOALLOC_MAX_PARTICLES bounds n: room for 2 counts per 256-particle tile (the
+// ranges use fewer), 256 KiB in all, resident on every GPU that loads the library until the process exits.
 // Every call shares that array and leaves the last call's counts in it.  No
-// entry needs clearing before a call (count_kernel writes every tile's counts
-// before scan_kernel reads them), but two calls whose work overlaps on the
+// entry needs clearing before a call (count_kernel writes every range's counts
+// before scatter_kernel reads them), but two calls whose work overlaps on the
 // GPU, on one stream or several, race on the array and corrupt each other.
 constexpr size_t NOALLOC_MAX_PARTICLES = 8u << 20;
 constexpr size_t NOALLOC_TILES = NOALLOC_MAX_PARTICLES / TILE;
@@ -269,11 +311,7 @@ int launch_partition_noalloc(const glisser_particles* in, const glisser_particle
         cudaMemsetAsync(n1, 0, sizeof(uint32_t), stream);
         return cudaGetLastError() == cudaSuccess ? GLISSER_OK : GLISSER_E_CUDA;
     }
-    uint32_t tiles = (uint32_t)((n + TILE - 1) / TILE);
-    count_kernel<<<tiles, TILE, 0, stream>>>(in->flags, (uint32_t)n, counts);
-    scan_kernel<<<1, SCAN_THREADS, 0, stream>>>(counts, tiles, n0, n1);
-    scatter_kernel<<<tiles, TILE, 0, stream>>>(*in, *out, (uint32_t)n, counts, n0, n1);
-    return cudaGetLastError() == cudaSuccess ? GLISSER_OK : GLISSER_E_CUDA;
+    return launch_two(in, out, (uint32_t)n, counts, n0, n1, stream);
 }
 
 }  // namespace glisser
