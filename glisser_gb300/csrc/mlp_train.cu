@@ -2,20 +2,28 @@
 // with hand-written forward/backward kernels (BF16 weights in, FP32
 // accumulation), and the device copy of the weights the drift reads.
 //
-// Training kernel layout: one CTA of 128 threads takes a tile of 128
-// samples, one per thread.  Each thread runs the forward pass of its sample
-// in the order of mlp_forward, the inputs and the hidden activations rounded
-// to the BF16 hi + lo pairs its products read (gradients straight through
-// the rounding), so the trained network is the one the drift evaluates; it
-// keeps the pre-activations of the second layer in registers, and runs the backward pass to the per-sample deltas, which it
-// writes to shared-memory tiles (rows padded to 33 floats: the row-per-thread
-// writes and the column reads are both bank-conflict free).  The weight
-// gradients are then sums over the tile's samples -- the FP32-accumulated
-// products of the stored activations and deltas -- computed with each thread
-// owning a fixed set of parameters, and written as one partial per CTA.  A
-// second kernel sums the partials in a fixed order (deterministic) and takes
-// the Adam step on the FP32 master weights; the next forward pass re-rounds
-// them to BF16.
+// Training kernel layout: one CTA takes a tile of 128 samples, four threads a
+// sample, each with a quarter of the hidden units.  The forward pass is
+// mlp_forward's, in its order, the inputs and the hidden activations rounded to
+// the BF16 hi + lo pairs its products read (gradients straight through the
+// rounding), so the trained network is the one the drift evaluates.
+// Activations and deltas go to shared-memory tiles; the weight gradients are
+// sums over the tile's samples -- the FP32-accumulated products of the stored
+// activations and deltas -- each computed by one thread in sample order and
+// written as one partial per CTA.  A second kernel sums the partials in CTA
+// order (deterministic) and takes the Adam step on the FP32 master weights; the
+// next forward pass re-rounds them to BF16.
+//
+// Bound: latency.  A minibatch of 16,384 is 128 CTAs, less than one an SM, so
+// a step is as long as one CTA's chain.  Four warps per scheduler fill one
+// another's waits, a row's activations are read once into registers, weight
+// rows come as 16-byte broadcasts, and the losses stay on the device until the
+// run ends (a copy to the host each step waited for it).  Every sum keeps its
+// order, so the results are, bit for bit, those of one thread a sample with two
+// 4-byte shared-memory reads per product, which took 48 us a step of 16,384; one
+// thread a sample with the reads vectorised 22.7 us; four threads a sample, W2's
+// sums in register tiles and each kernel's start-up under the one before it
+// (launch_early) 12.9 us.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -28,8 +36,10 @@ namespace glisser {
 
 namespace {
 
-constexpr int TT = 128;                  // samples per training tile (one per thread)
-constexpr int HP = MLP_H + 1;            // padded activation row
+constexpr int TT = 128;                  // samples per training tile
+constexpr int TPS = 4;                   // threads per sample, each a quarter of the hidden units
+constexpr int UPT = MLP_H / TPS;         // hidden units per thread
+constexpr int HP = MLP_H + 4;            // padded activation row: 16-byte aligned, float4 accesses free of bank conflicts
 constexpr int PART = MLP_NPARAM + 1;     // per-CTA partial: gradients, then the loss sum
 constexpr int SM_WEIGHTS = MLP_H * 4 + MLP_H + MLP_H * MLP_H + MLP_H + MLP_H + 4;
 constexpr int SM_FLOATS = SM_WEIGHTS + 4 * TT * HP + TT * 4 + 2 * TT;
@@ -111,10 +121,15 @@ __device__ __forceinline__ float dsilu(float a)
     return s * fmaf(a, 1.0f - s, 1.0f);
 }
 
-__global__ void __launch_bounds__(TT) grad_kernel(const float* __restrict__ params, const TrainArgs a,
-                                                  float* __restrict__ partials)
+// The four floats of a row's group q as an array.
+__device__ __forceinline__ void unpack4(const float4 v, float* f)
 {
-    extern __shared__ float sm[];
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+}
+
+__global__ void __launch_bounds__(TT * TPS) grad_kernel(const float* params, const TrainArgs a, float* partials)
+{
+    extern __shared__ __align__(16) float sm[];
     float* W1 = sm;                       // [MLP_H][4]
     float* B1 = W1 + MLP_H * 4;
     float* W2 = B1 + MLP_H;               // [MLP_H][MLP_H]
@@ -129,131 +144,219 @@ __global__ void __launch_bounds__(TT) grad_kernel(const float* __restrict__ para
     float* DY = X + TT * 4;               // [TT] output deltas
     float* LS = DY + TT;                  // [TT] squared errors
 
-    const int t = threadIdx.x;
-    for (int q = t; q < MLP_H * 4; q += TT) {
+    // thread t: sample i of the tile, hidden units u0 .. u0 + UPT - 1 (a warp's
+    // threads share theirs, so that weight rows are broadcasts)
+    const int t = threadIdx.x, i = t % TT, part = t / TT, u0 = part * UPT;
+    float f0 = 0, f1 = 0, f2 = 0, tg = 0;
+    bool valid = false;
+    if (part == 0) {
+        // this thread's sample, on its way while the weights are staged
+        const uint32_t gi = blockIdx.x * TT + i;
+        valid = gi < a.batch;
+        if (valid) {
+            const uint32_t idx = a.sequential ? gi : mix32(a.seed ^ ((uint64_t)a.step << 32) ^ gi) % a.n;
+            f0 = a.feat[3 * (size_t)idx];
+            f1 = a.feat[3 * (size_t)idx + 1];
+            f2 = a.feat[3 * (size_t)idx + 2];
+            tg = a.target[idx];
+        }
+    }
+    // the parameters of the update before this step (and its partials read)
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    for (int q = t; q < MLP_H * 4; q += TT * TPS) {
         const int j = q >> 2, k = q & 3;
         W1[q] = k < MLP_IN ? bf16_round(params[MLP_OFF_W1 + j * MLP_IN + k]) : 0.0f;
     }
-    for (int q = t; q < MLP_H * MLP_H; q += TT) W2[q] = bf16_round(params[MLP_OFF_W2 + q]);
+    for (int q = t; q < MLP_H * MLP_H; q += TT * TPS) W2[q] = bf16_round(params[MLP_OFF_W2 + q]);
     if (t < MLP_H) {
         B1[t] = params[MLP_OFF_B1 + t];
         B2[t] = params[MLP_OFF_B2 + t];
         W3[t] = bf16_round(params[MLP_OFF_W3 + t]);
     }
     if (t == 0) B3[0] = params[MLP_OFF_B3];
+    float tn = 0;
+    if (part == 0) {
+        valid = valid && isfinite(tg) && isfinite(f0) && isfinite(f1) && isfinite(f2);
+        float x0 = 0, x1 = 0, x2 = 0;
+        if (valid) {
+            // the inputs as the first layer reads them (BF16 hi + lo)
+            x0 = bf16_split_sum((f0 - a.norm.in_mean[0]) * a.norm.in_scale[0]);
+            x1 = bf16_split_sum((f1 - a.norm.in_mean[1]) * a.norm.in_scale[1]);
+            x2 = bf16_split_sum((f2 - a.norm.in_mean[2]) * a.norm.in_scale[2]);
+            tn = (tg - a.norm.out_mean) / a.norm.out_scale;
+        }
+        *reinterpret_cast<float4*>(X + 4 * i) = make_float4(x0, x1, x2, 0.0f);
+    }
     __syncthreads();
-
-    // this thread's sample
-    const uint32_t gi = blockIdx.x * TT + t;
-    bool valid = gi < a.batch;
-    float f0 = 0, f1 = 0, f2 = 0, tg = 0;
-    if (valid) {
-        const uint32_t idx = a.sequential ? gi : mix32(a.seed ^ ((uint64_t)a.step << 32) ^ gi) % a.n;
-        f0 = a.feat[3 * (size_t)idx];
-        f1 = a.feat[3 * (size_t)idx + 1];
-        f2 = a.feat[3 * (size_t)idx + 2];
-        tg = a.target[idx];
-        valid = isfinite(tg) && isfinite(f0) && isfinite(f1) && isfinite(f2);
-    }
-    float x0 = 0, x1 = 0, x2 = 0, tn = 0;
-    if (valid) {
-        // the inputs as the first layer reads them (BF16 hi + lo)
-        x0 = bf16_split_sum((f0 - a.norm.in_mean[0]) * a.norm.in_scale[0]);
-        x1 = bf16_split_sum((f1 - a.norm.in_mean[1]) * a.norm.in_scale[1]);
-        x2 = bf16_split_sum((f2 - a.norm.in_mean[2]) * a.norm.in_scale[2]);
-        tn = (tg - a.norm.out_mean) / a.norm.out_scale;
-    }
 
     // forward, in the order of mlp_forward
-    float* h1 = H1 + t * HP;
-    float* h2 = H2 + t * HP;
-#pragma unroll 4
-    for (int j = 0; j < MLP_H; j++) {
-        float z = B1[j];
-        z = fmaf(W1[4 * j], x0, z);
-        z = fmaf(W1[4 * j + 1], x1, z);
-        z = fmaf(W1[4 * j + 2], x2, z);
-        h1[j] = bf16_split_sum(z * mlp_sigmoid(z));   // as the hidden layer reads it; straight-through below
+    const float4* W1v = reinterpret_cast<const float4*>(W1);
+    const float4* W2v = reinterpret_cast<const float4*>(W2);
+    float4* h1row = reinterpret_cast<float4*>(H1 + i * HP);
+    float4* h2row = reinterpret_cast<float4*>(H2 + i * HP);
+    float4* d1row = reinterpret_cast<float4*>(D1 + i * HP);
+    float4* d2row = reinterpret_cast<float4*>(D2 + i * HP);
+    const float4 x = *reinterpret_cast<const float4*>(X + 4 * i);
+    float ds1[UPT];                       // SiLU's derivative at this thread's layer-1 units
+    {
+        float h[UPT];
+#pragma unroll
+        for (int c = 0; c < UPT; c++) {
+            const float4 w = W1v[u0 + c];
+            float z = B1[u0 + c];
+            z = fmaf(w.x, x.x, z);
+            z = fmaf(w.y, x.y, z);
+            z = fmaf(w.z, x.z, z);
+            h[c] = bf16_split_sum(z * mlp_sigmoid(z));   // as the hidden layer reads it; straight-through below
+            ds1[c] = dsilu(z);
+        }
+#pragma unroll
+        for (int q = 0; q < UPT / 4; q++)
+            h1row[u0 / 4 + q] = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
     }
-    float a2[MLP_H];
-    float y = B3[0];
+    __syncthreads();
+    float ds2[UPT];
+    {
+        float h[MLP_H], z[UPT];
 #pragma unroll
-    for (int j = 0; j < MLP_H; j++) {
-        float z = B2[j];
+        for (int q = 0; q < MLP_H / 4; q++) unpack4(h1row[q], h + 4 * q);
 #pragma unroll
-        for (int k = 0; k < MLP_H; k++) z = fmaf(W2[j * MLP_H + k], h1[k], z);
-        a2[j] = z;
-        const float hv = z * mlp_sigmoid(z);
-        h2[j] = hv;
-        y = fmaf(W3[j], hv, y);
+        for (int c = 0; c < UPT; c++) z[c] = B2[u0 + c];
+#pragma unroll
+        for (int q = 0; q < MLP_H / 4; q++) {
+#pragma unroll
+            for (int c = 0; c < UPT; c++) {
+                const float4 w = W2v[(u0 + c) * (MLP_H / 4) + q];
+                z[c] = fmaf(w.x, h[4 * q], z[c]);
+                z[c] = fmaf(w.y, h[4 * q + 1], z[c]);
+                z[c] = fmaf(w.z, h[4 * q + 2], z[c]);
+                z[c] = fmaf(w.w, h[4 * q + 3], z[c]);
+            }
+        }
+        float hv[UPT];
+#pragma unroll
+        for (int c = 0; c < UPT; c++) {
+            hv[c] = z[c] * mlp_sigmoid(z[c]);
+            ds2[c] = dsilu(z[c]);
+        }
+#pragma unroll
+        for (int q = 0; q < UPT / 4; q++)
+            h2row[u0 / 4 + q] = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
     }
-    const float err = valid ? y - tn : 0.0f;
-    const float dy = 2.0f * err * a.inv_batch;
-    LS[t] = err * err;
-    DY[t] = dy;
-    X[4 * t] = x0;
-    X[4 * t + 1] = x1;
-    X[4 * t + 2] = x2;
-
-    // backward to the per-sample deltas
-    float* d2 = D2 + t * HP;
-    float* d1 = D1 + t * HP;
+    __syncthreads();
+    if (part == 0) {
+        float y = B3[0];
 #pragma unroll
-    for (int j = 0; j < MLP_H; j++) d2[j] = dy * W3[j] * dsilu(a2[j]);
-#pragma unroll 4
-    for (int k = 0; k < MLP_H; k++) {
-        float z = B1[k];
-        z = fmaf(W1[4 * k], x0, z);
-        z = fmaf(W1[4 * k + 1], x1, z);
-        z = fmaf(W1[4 * k + 2], x2, z);
-        float dh = 0.0f;
-#pragma unroll 8
-        for (int j = 0; j < MLP_H; j++) dh = fmaf(W2[j * MLP_H + k], d2[j], dh);
-        d1[k] = dh * dsilu(z);
+        for (int q = 0; q < MLP_H / 4; q++) {
+            float hv[4];
+            unpack4(h2row[q], hv);
+#pragma unroll
+            for (int c = 0; c < 4; c++) y = fmaf(W3[4 * q + c], hv[c], y);
+        }
+        const float err = valid ? y - tn : 0.0f;
+        LS[i] = err * err;
+        DY[i] = 2.0f * err * a.inv_batch;
     }
     __syncthreads();
 
-    // parameter gradients summed over the tile
-    float* out = partials + (size_t)blockIdx.x * PART;
+    // backward to the per-sample deltas
     {
-        // W2: thread t owns row j = t / 4, columns 8 (t % 4) .. + 7
-        const int j = t >> 2, kb = (t & 3) * 8;
-        float acc[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-        for (int i = 0; i < TT; i++) {
-            const float d = D2[i * HP + j];
+        const float dy = DY[i];
+        float d[UPT];
 #pragma unroll
-            for (int q = 0; q < 8; q++) acc[q] = fmaf(d, H1[i * HP + kb + q], acc[q]);
+        for (int c = 0; c < UPT; c++) d[c] = dy * W3[u0 + c] * ds2[c];
+#pragma unroll
+        for (int q = 0; q < UPT / 4; q++)
+            d2row[u0 / 4 + q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
+    }
+    __syncthreads();
+    {
+        float d[MLP_H], dh[UPT];
+#pragma unroll
+        for (int q = 0; q < MLP_H / 4; q++) unpack4(d2row[q], d + 4 * q);
+#pragma unroll
+        for (int c = 0; c < UPT; c++) dh[c] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < MLP_H; j++) {
+#pragma unroll
+            for (int q = 0; q < UPT / 4; q++) {
+                const float4 w = W2v[j * (MLP_H / 4) + u0 / 4 + q];
+                dh[4 * q] = fmaf(w.x, d[j], dh[4 * q]);
+                dh[4 * q + 1] = fmaf(w.y, d[j], dh[4 * q + 1]);
+                dh[4 * q + 2] = fmaf(w.z, d[j], dh[4 * q + 2]);
+                dh[4 * q + 3] = fmaf(w.w, d[j], dh[4 * q + 3]);
+            }
         }
 #pragma unroll
-        for (int q = 0; q < 8; q++) out[MLP_OFF_W2 + j * MLP_H + kb + q] = acc[q];
+        for (int q = 0; q < UPT / 4; q++)
+            d1row[u0 / 4 + q] = make_float4(dh[4 * q] * ds1[4 * q], dh[4 * q + 1] * ds1[4 * q + 1],
+                                            dh[4 * q + 2] * ds1[4 * q + 2], dh[4 * q + 3] * ds1[4 * q + 3]);
     }
-    if (t < MLP_H * MLP_IN) {
-        const int j = t / MLP_IN, k = t % MLP_IN;
+    __syncthreads();
+
+    // parameter gradients summed over the tile, each by one thread in sample order
+    float* out = partials + (size_t)blockIdx.x * PART;
+    {
+        // W2 on the first four warps, one a scheduler: thread t owns rows 2 (t / 8) and
+        // the next, columns 4 (t % 8) .. + 3 (eight products for two reads); the
+        // others' sums on the warps beside them
+        if (t < 128) {
+            const int j = (t >> 3) * 2, k = (t & 7) * 4;
+            float acc[2][4] = { { 0, 0, 0, 0 }, { 0, 0, 0, 0 } };
+#pragma unroll 8
+            for (int n = 0; n < TT; n++) {
+                const float2 d = *reinterpret_cast<const float2*>(D2 + n * HP + j);
+                float h[4];
+                unpack4(*reinterpret_cast<const float4*>(H1 + n * HP + k), h);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    acc[0][c] = fmaf(d.x, h[c], acc[0][c]);
+                    acc[1][c] = fmaf(d.y, h[c], acc[1][c]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                out[MLP_OFF_W2 + j * MLP_H + k + c] = acc[0][c];
+                out[MLP_OFF_W2 + (j + 1) * MLP_H + k + c] = acc[1][c];
+            }
+            return;
+        }
+    }
+    const int r = t - 128;
+    if (r < MLP_H * MLP_IN) {
+        const int j = r / MLP_IN, k = r % MLP_IN;
         float acc = 0;
-        for (int i = 0; i < TT; i++) acc = fmaf(D1[i * HP + j], X[4 * i + k], acc);
-        out[MLP_OFF_W1 + t] = acc;
-    } else {
-        const int j = t - MLP_H * MLP_IN;
+#pragma unroll 16
+        for (int n = 0; n < TT; n++) acc = fmaf(D1[n * HP + j], X[4 * n + k], acc);
+        out[MLP_OFF_W1 + r] = acc;
+    } else if (r < MLP_H * MLP_IN + MLP_H) {
+        const int j = r - MLP_H * MLP_IN;
         float acc = 0;
-        for (int i = 0; i < TT; i++) acc += D1[i * HP + j];
+#pragma unroll 16
+        for (int n = 0; n < TT; n++) acc += D1[n * HP + j];
         out[MLP_OFF_B1 + j] = acc;
-    }
-    if (t < MLP_H) {
+    } else if (r < MLP_H * MLP_IN + 2 * MLP_H) {
+        const int j = r - MLP_H * MLP_IN - MLP_H;
         float acc = 0;
-        for (int i = 0; i < TT; i++) acc += D2[i * HP + t];
-        out[MLP_OFF_B2 + t] = acc;
-    } else if (t < 2 * MLP_H) {
-        const int j = t - MLP_H;
+#pragma unroll 16
+        for (int n = 0; n < TT; n++) acc += D2[n * HP + j];
+        out[MLP_OFF_B2 + j] = acc;
+    } else if (r < MLP_H * MLP_IN + 3 * MLP_H) {
+        const int j = r - MLP_H * MLP_IN - 2 * MLP_H;
         float acc = 0;
-        for (int i = 0; i < TT; i++) acc = fmaf(DY[i], H2[i * HP + j], acc);
+#pragma unroll 16
+        for (int n = 0; n < TT; n++) acc = fmaf(DY[n], H2[n * HP + j], acc);
         out[MLP_OFF_W3 + j] = acc;
-    } else if (t == 2 * MLP_H) {
+    } else if (r == MLP_H * MLP_IN + 3 * MLP_H) {
         float acc = 0;
-        for (int i = 0; i < TT; i++) acc += DY[i];
+#pragma unroll 16
+        for (int n = 0; n < TT; n++) acc += DY[n];
         out[MLP_OFF_B3] = acc;
-    } else if (t == 2 * MLP_H + 1) {
+    } else if (r == MLP_H * MLP_IN + 4 * MLP_H) {
         float acc = 0;
-        for (int i = 0; i < TT; i++) acc += LS[i];
+#pragma unroll 16
+        for (int n = 0; n < TT; n++) acc += LS[n];
         out[MLP_NPARAM] = acc;
     }
 }
@@ -263,18 +366,32 @@ struct AdamArgs {
     uint32_t apply;        // 0: only sum the partials into `grad`
 };
 
-// Sums the CTA partials in CTA order; then (apply) one Adam step.  grad
-// (optional) receives the summed gradients and, at index MLP_NPARAM, the
-// mean loss.
-__global__ void adam_kernel(float* params, float* m, float* v, const float* __restrict__ partials, uint32_t nblk,
-                            AdamArgs a, float* grad)
+// Sums the CTA partials in CTA order (the reads of a group of them in flight at
+// once); then (apply) one Adam step.  grad (optional) receives the summed
+// gradients, loss (optional) the mean loss.
+constexpr int ADAM_THREADS = 32;     // small CTAs: the 1,218 sums spread over the SMs
+constexpr int ADAM_GROUP = 64;
+
+__global__ void __launch_bounds__(ADAM_THREADS)
+    adam_kernel(float* params, float* m, float* v, const float* partials, uint32_t nblk, AdamArgs a,
+                float* grad, float* loss)
 {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if (p > (uint32_t)MLP_NPARAM) return;
     float g = 0;
-    for (uint32_t b = 0; b < nblk; b++) g += partials[(size_t)b * PART + p];
+    uint32_t b = 0;
+    for (; b + ADAM_GROUP <= nblk; b += ADAM_GROUP) {
+        float x[ADAM_GROUP];
+#pragma unroll
+        for (int k = 0; k < ADAM_GROUP; k++) x[k] = partials[(size_t)(b + k) * PART + p];
+#pragma unroll
+        for (int k = 0; k < ADAM_GROUP; k++) g += x[k];
+    }
+    for (; b < nblk; b++) g += partials[(size_t)b * PART + p];
     if (p == (uint32_t)MLP_NPARAM) {
-        if (grad) grad[p] = g * a.inv_batch;
+        if (loss) *loss = g * a.inv_batch;
         return;
     }
     if (grad) grad[p] = g;
@@ -321,6 +438,25 @@ __global__ void drift_states_kernel(glisser_particles pa, uint32_t n, double dt,
     pa.vx[i] = vx; pa.vy[i] = vy; pa.vz[i] = vz;
     if (evals) evals[i] = d.evals;
     if (flags) flags[i] = d.flags;
+}
+
+// A launch that may begin before the kernel ahead of it in the stream has ended
+// (programmatic dependent launch): the training kernels wait for that end
+// themselves, so only their start-up overlaps.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kern)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t stream, A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, args...);
 }
 
 uint32_t bf16_bits_round(float x)
@@ -565,8 +701,8 @@ void MlpTrainer::grad_launch(const float* feat, const float* target, uint32_t n,
     a.seed = seed;
     a.inv_batch = 1.0f / (float)batch;
     a.norm = norm;
-    grad_kernel<<<blocks, TT, SM_FLOATS * sizeof(float), stream_>>>(d_params_, a, d_partials_);
-    check(cudaGetLastError(), "grad_kernel");
+    check(launch_early(grad_kernel, blocks, TT * TPS, SM_FLOATS * sizeof(float), stream_, (const float*)d_params_, a,
+                       d_partials_), "grad_kernel");
 }
 
 void MlpTrainer::train(int steps, int batch, float lr, float lr_min, uint64_t seed, float* losses)
@@ -575,7 +711,12 @@ void MlpTrainer::train(int steps, int batch, float lr, float lr_min, uint64_t se
     if (steps < 0 || batch < TT || batch % TT != 0) throw std::invalid_argument("train: batch must be a multiple of 128");
     const uint32_t blocks = (uint32_t)(batch / TT);
     ensure_partials(blocks);
-    std::vector<float> hl(losses ? steps : 0);
+    // the losses of the run, one per step
+    struct DeviceFloats {
+        float* p = nullptr;
+        ~DeviceFloats() { cudaFree(p); }
+    } dl;
+    if (losses && steps > 0) check(cudaMalloc(&dl.p, (size_t)steps * sizeof(float)), "losses");
     const float b1 = 0.9f, b2 = 0.999f;
     for (int s = 0; s < steps; s++) {
         grad_launch(d_feat_, d_target_, (uint32_t)n_, (uint32_t)batch, false, seed, (uint32_t)s, blocks);
@@ -590,15 +731,12 @@ void MlpTrainer::train(int steps, int batch, float lr, float lr_min, uint64_t se
         a.bc2 = (float)(1.0 - std::pow((double)b2, adam_t_));
         a.inv_batch = 1.0f / (float)batch;
         a.apply = 1;
-        adam_kernel<<<(MLP_NPARAM + 1 + 127) / 128, 128, 0, stream_>>>(d_params_, d_m_, d_v_, d_partials_, blocks, a,
-                                                                      losses ? d_loss_ : nullptr);
-        check(cudaGetLastError(), "adam_kernel");
-        if (losses) {
-            check(cudaMemcpyAsync(&hl[s], d_loss_ + MLP_NPARAM, sizeof(float), cudaMemcpyDeviceToHost, stream_), "loss");
-        }
+        check(launch_early(adam_kernel, MLP_NPARAM / ADAM_THREADS + 1, ADAM_THREADS, 0, stream_, d_params_, d_m_, d_v_,
+                           (const float*)d_partials_, blocks, a, (float*)nullptr, dl.p ? dl.p + s : (float*)nullptr),
+              "adam_kernel");
     }
     check(cudaStreamSynchronize(stream_), "training");
-    if (losses) std::memcpy(losses, hl.data(), steps * sizeof(float));
+    if (dl.p) check(cudaMemcpy(losses, dl.p, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost), "losses");
     check(cudaMemcpy(params_.data(), d_params_, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost), "parameters");
     dev_stale_ = true;
 }
@@ -619,9 +757,9 @@ void MlpTrainer::gradients(const float* feat, const float* target, size_t n, flo
         std::memset(&a, 0, sizeof a);
         a.inv_batch = 1.0f / (float)n;
         a.apply = 0;
-        adam_kernel<<<(MLP_NPARAM + 1 + 127) / 128, 128, 0, stream_>>>(d_params_, d_m_, d_v_, d_partials_, blocks, a,
-                                                                      d_loss_);
-        check(cudaGetLastError(), "adam_kernel");
+        check(launch_early(adam_kernel, MLP_NPARAM / ADAM_THREADS + 1, ADAM_THREADS, 0, stream_, d_params_, d_m_, d_v_,
+                           (const float*)d_partials_, blocks, a, d_loss_, d_loss_ + MLP_NPARAM),
+              "adam_kernel");
         std::vector<float> g(MLP_NPARAM + 1);
         check(cudaMemcpyAsync(g.data(), d_loss_, g.size() * sizeof(float), cudaMemcpyDeviceToHost, stream_), "grad");
         check(cudaStreamSynchronize(stream_), "gradients");
