@@ -57,9 +57,10 @@ __global__ void __launch_bounds__(CTA, (LEARNED ? GLISSER_BATCHED_THREADS_PER_SM
 
 template <int NP, int CTA, int PPT, bool LEARNED, bool KICK64>
 cudaError_t launch_batched_t(const Common& p, const BatchSystems& sys, const BatchItem* items,
-                             const uint32_t* n_items, uint32_t* queue, uint32_t grid, size_t smem,
+                             const uint32_t* n_items, uint32_t* queue, const BatchShape& shape, size_t smem,
                              cudaStream_t stream)
 {
+    uint32_t grid = shape.grid;
     auto kern = batched_kernel<NP, CTA, PPT, LEARNED, KICK64>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -69,6 +70,10 @@ cudaError_t launch_batched_t(const Common& p, const BatchSystems& sys, const Bat
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, CTA, smem);
         grid = (uint32_t)(sms * (per > 0 ? per : 1));
+        // with fewer items than CTAs, which CTAs pop one is a matter of chance, and an
+        // SM may hold several of them while others hold none: one CTA per item is
+        // spread evenly (16 systems, 9,000 particles x 256 steps: 1.86 -> 0.64 ms)
+        if (shape.items && shape.items < grid) grid = shape.items;
     }
     kern<<<grid, CTA, smem, stream>>>(p, sys, items, n_items, queue);
     return cudaGetLastError();
@@ -80,14 +85,13 @@ cudaError_t launch_batched_np(const Common& p, const BatchSystems& sys, const Ba
                               cudaStream_t stream)
 {
     const int key = shape.cta * 10 + shape.ppt;
-    const uint32_t g = shape.grid;
     switch (key) {
-    case 641: return launch_batched_t<NP, 64, 1, LEARNED, KICK64>(p, sys, items, n_items, queue, g, smem, stream);
-    case 642: return launch_batched_t<NP, 64, 2, LEARNED, KICK64>(p, sys, items, n_items, queue, g, smem, stream);
-    case 1281: return launch_batched_t<NP, 128, 1, LEARNED, KICK64>(p, sys, items, n_items, queue, g, smem, stream);
-    case 1282: return launch_batched_t<NP, 128, 2, LEARNED, KICK64>(p, sys, items, n_items, queue, g, smem, stream);
-    case 2561: return launch_batched_t<NP, 256, 1, LEARNED, KICK64>(p, sys, items, n_items, queue, g, smem, stream);
-    case 2562: return launch_batched_t<NP, 256, 2, LEARNED, KICK64>(p, sys, items, n_items, queue, g, smem, stream);
+    case 641: return launch_batched_t<NP, 64, 1, LEARNED, KICK64>(p, sys, items, n_items, queue, shape, smem, stream);
+    case 642: return launch_batched_t<NP, 64, 2, LEARNED, KICK64>(p, sys, items, n_items, queue, shape, smem, stream);
+    case 1281: return launch_batched_t<NP, 128, 1, LEARNED, KICK64>(p, sys, items, n_items, queue, shape, smem, stream);
+    case 1282: return launch_batched_t<NP, 128, 2, LEARNED, KICK64>(p, sys, items, n_items, queue, shape, smem, stream);
+    case 2561: return launch_batched_t<NP, 256, 1, LEARNED, KICK64>(p, sys, items, n_items, queue, shape, smem, stream);
+    case 2562: return launch_batched_t<NP, 256, 2, LEARNED, KICK64>(p, sys, items, n_items, queue, shape, smem, stream);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -569,7 +569,9 @@ void Ensemble::enqueue(int par, int starter)
     ho.borderline = d.d_evals + 1;
     ho.learned = d.d_evals + 2;
     ho.wide = d.d_evals + 3;
-    int rc = launch_batched(&d.pa, sy, d.d_items[par], d.d_nitems[par], d.d_ctr + 2, npl_, len_, &sp, &ho, shape_,
+    BatchShape shape = shape_;
+    shape.items = (uint32_t)tile_first_.size();
+    int rc = launch_batched(&d.pa, sy, d.d_items[par], d.d_nitems[par], d.d_ctr + 2, npl_, len_, &sp, &ho, shape,
                             d.stream);
     if (rc != GLISSER_OK) throw CudaError(std::string("batched launch failed: ") + timeblock_error());
     ck(cudaMemcpyAsync(d.h_ctr, d.d_ctr, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, d.stream), "counters");

@@ -60,7 +60,8 @@ struct BatchItem {
 struct BatchShape {
     int cta;                // threads per CTA: 64, 128 or 256
     int ppt;                // particles per thread: 1 or 2
-    uint32_t grid;          // persistent CTAs (0: one wave at full occupancy)
+    uint32_t grid;          // persistent CTAs (0: one wave at full occupancy, at most `items` CTAs)
+    uint32_t items = 0;     // the most work items a block can have (0: not known)
 };
 
 int launch_batched(const glisser_particles* pa, const BatchSystems& sys, const BatchItem* items,
