@@ -179,11 +179,13 @@ __device__ __forceinline__ bool ff_lt(ff a, ff b) { return a.hi < b.hi || (a.hi 
 
 __device__ __forceinline__ ff ff_scale(ff a, float pow2) { return { a.hi * pow2, a.lo * pow2 }; }   // exact
 
-// 1/3, 1/6, 1/12, -1/24, -1/120 and 1/720 as float-floats (hi the nearest float, lo
+// 1/3, 1/6, 1/12, 1/20, 1/30, -1/24, -1/120 and 1/720 as float-floats (hi the nearest float, lo
 // the nearest float to the remainder: within 1.1e-15 relative)
 __device__ __forceinline__ ff ff_sixth() { return { 1.0f / 6.0f, -4.9670538e-09f }; }
 __device__ __forceinline__ ff ff_third() { return { 1.0f / 3.0f, -9.9341077e-09f }; }
 __device__ __forceinline__ ff ff_twelfth() { return { 1.0f / 12.0f, -2.4835269e-09f }; }
+__device__ __forceinline__ ff ff_20th() { return { 1.0f / 20.0f, -7.45058071e-10f }; }
+__device__ __forceinline__ ff ff_30th() { return { 1.0f / 30.0f, -1.73846881e-09f }; }
 __device__ __forceinline__ ff ff_neg_24th() { return { -1.0f / 24.0f, 1.2417635e-09f }; }
 __device__ __forceinline__ ff ff_neg_120th() { return { -1.0f / 120.0f, 4.346172e-10f }; }
 __device__ __forceinline__ ff ff_720th() { return { 1.0f / 720.0f, -3.3631094e-11f }; }

@@ -633,12 +633,33 @@ __device__ __forceinline__ DriftInvariants drift_invariants(double rx, double ry
     return q;
 }
 
-// Drifts (r, v) by dt about a central mass mu, given the drift's invariants
-// q.  r2 = |r|^2 and rinv = 1/|r| come in for the state and go out for the
-// new position, both taken from the new position vector itself (its length
-// enters the energy alpha = 2 mu / r0 - v^2 of the next drift, where near
-// pericentre of an eccentric orbit any inconsistency with the vector is
-// magnified).  tol_dt = the residual tolerance times dt (KEP_TOL * dt by
+// Applies the f and g functions of a drift by dt, given its G-functions at the
+// root.  r2 = |r|^2 and rinv = 1/|r| go out for the new position, both taken from
+// the new position vector itself (its length enters the energy alpha =
+// 2 mu / r0 - v^2 of the next drift, where near pericentre of an eccentric orbit
+// any inconsistency with the vector is magnified).
+__device__ __forceinline__ void drift_apply(double& rx, double& ry, double& rz, double& vx, double& vy, double& vz,
+                                            double& r2_out, double& rinv_out, const GFun& g, double mu_r, double dt,
+                                            double mu)
+{
+    const double g3 = g.g3, g2 = g.g2, g1 = g.g1;
+    double ff = fma(-mu_r, g2, 1.0);
+    double gg = fma(-mu, g3, dt);
+    double nrx = fma(ff, rx, gg * vx), nry = fma(ff, ry, gg * vy), nrz = fma(ff, rz, gg * vz);
+    const double nr2 = fma(nrx, nrx, fma(nry, nry, nrz * nrz));
+    const double nrinv = rsqrt_lean(nr2);
+    double fd = -mu_r * g1 * nrinv;
+    double gd = fma(-mu * g2, nrinv, 1.0);
+    double nvx = fma(fd, rx, gd * vx), nvy = fma(fd, ry, gd * vy), nvz = fma(fd, rz, gd * vz);
+    rx = nrx; ry = nry; rz = nrz;
+    vx = nvx; vy = nvy; vz = nvz;
+    r2_out = nr2;
+    rinv_out = nrinv;
+}
+
+// Solves Kepler's equation of a drift by dt about a central mass mu for the
+// G-functions at the root (the last evaluation's when not converged), given the
+// drift's invariants q and rinv = 1/|r|.  tol_dt = the residual tolerance times dt (KEP_TOL * dt by
 // default).  `starter` picks the classic or the series rule: the tenth-order
 // series while tau^2 < SERIES_TAU2_MAX, else the FP32 Kepler pre-solve for
 // bound orbits and the classic starter for unbound ones.  LEARNED (weights
@@ -651,11 +672,9 @@ __device__ __forceinline__ DriftInvariants drift_invariants(double rx, double ry
 // is the restart, for the bounded Laguerre iteration that is every starter's
 // last resort.
 template <bool LEARNED, int NET_ROWS = MLP_ROWS, int NET_QU = 1>
-__device__ __forceinline__ DriftResult kepler_drift(double& rx, double& ry, double& rz, double& vx, double& vy, double& vz,
-                                                   double& r2_io, double& rinv_io, const DriftInvariants& q, double dt,
-                                                   double mu, int starter, const MlpDev* mlp, double tol_dt)
+__device__ __forceinline__ DriftResult kepler_solve(GFun& g, double rinv, const DriftInvariants& q, double dt, double mu,
+                                                   int starter, const MlpDev* mlp, double tol_dt)
 {
-    const double rinv = rinv_io;
     const double r0 = q.r0, u = q.u, mu_r = q.mu_r, alpha = q.alpha, T = q.T;
     DriftResult res;
     res.flags = __double_as_longlong(alpha) <= 0 ? 0x08 : 0;   // alpha <= 0 (or negative NaN), integer pipe
@@ -678,7 +697,6 @@ __device__ __forceinline__ DriftResult kepler_drift(double& rx, double& ry, doub
         else s = starter_classic(dt, r0, rinv, mu, alpha, u);
     }
     const double tol = tol_dt;
-    GFun g;
     double ds = 0;
     bool ok = kepler_newton(s, dt, r0, u, mu, alpha, tol, q.tau2 < SMALL_STEP_TAU2, g, ds, res.evals);
     if constexpr (LEARNED) {
@@ -689,32 +707,20 @@ __device__ __forceinline__ DriftResult kepler_drift(double& rx, double& ry, doub
     if (!ok) ok = kepler_laguerre(s, dt, r0, u, mu, alpha, tol, g, ds, res.evals);
     if (!ok) res.flags |= 0x04;
     res.net = net;
-    // g: the G-functions at the root (the last evaluation's when not converged)
-    const double g3 = g.g3, g2 = g.g2, g1 = g.g1;
-
-    double ff = fma(-mu_r, g2, 1.0);
-    double gg = fma(-mu, g3, dt);
-    double nrx = fma(ff, rx, gg * vx), nry = fma(ff, ry, gg * vy), nrz = fma(ff, rz, gg * vz);
-    const double nr2 = fma(nrx, nrx, fma(nry, nry, nrz * nrz));
-    const double nrinv = rsqrt_lean(nr2);
-    double fd = -mu_r * g1 * nrinv;
-    double gd = fma(-mu * g2, nrinv, 1.0);
-    double nvx = fma(fd, rx, gd * vx), nvy = fma(fd, ry, gd * vy), nvz = fma(fd, rz, gd * vz);
-    rx = nrx; ry = nry; rz = nrz;
-    vx = nvx; vy = nvy; vz = nvz;
-    r2_io = nr2;
-    rinv_io = nrinv;
     return res;
 }
 
-// The same drift for a single particle, its invariants formed here.
+// One drift of a state.
 template <bool LEARNED>
 __device__ __forceinline__ DriftResult kepler_drift(double& rx, double& ry, double& rz, double& vx, double& vy, double& vz,
                                                    double& r2_io, double& rinv_io, double dt, double mu, int starter,
                                                    const MlpDev* mlp, double tol_dt)
 {
     const DriftInvariants q = drift_invariants(rx, ry, rz, vx, vy, vz, r2_io, rinv_io, dt, mu);
-    return kepler_drift<LEARNED>(rx, ry, rz, vx, vy, vz, r2_io, rinv_io, q, dt, mu, starter, mlp, tol_dt);
+    GFun g;
+    const DriftResult res = kepler_solve<LEARNED>(g, rinv_io, q, dt, mu, starter, mlp, tol_dt);
+    drift_apply(rx, ry, rz, vx, vy, vz, r2_io, rinv_io, g, q.mu_r, dt, mu);
+    return res;
 }
 
 }  // namespace glisser

@@ -330,12 +330,12 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                 ff gx = { 0.0f, 0.0f }, gy = { 0.0f, 0.0f }, gz = { 0.0f, 0.0f };
                 // tau^2 / 2 in FP32 first: a wide drift costs the small-step one five instructions
                 const float q3 = sh.muh.hi * fri[k].hi * (fri[k].hi * fri[k].hi);
-                bool small = p.starter != STARTER_CLASSIC && q3 < 0.5f * SMALL_DRIFT_TAU2;
-                if (small) {
+                int tier = DRIFT_GENERAL;
+                if (p.starter != STARTER_CLASSIC && q3 < 0.5f * SMALL_DRIFT_TAU2) {
                     ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
-                    small = small_drift(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
+                    tier = small_drift<false>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
                 }
-                if (small) {
+                if (tier == DRIFT_SMALL) {
                     // r' = r + dt v + ((f - 1) r + (g - dt) v): dt v in FP64, the rest a
                     // float-float correction
                     const ff cx = ff_norm(ff_add_u(ff_mul_u(sd.f1, fx[k]), ff_mul_u(sd.gdt, wx)));
@@ -366,15 +366,31 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                         rinv[k] = rsqrt_lean(r2[k]);
                         general[k] = true;
                     }
-                    const DriftInvariants q =
-                        drift_invariants(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], p.dt, mu);
-                    DriftResult d = kepler_drift<LEARNED, NET_ROWS, NET_QU>(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k],
-                                                                             r2[k], rinv[k], q, p.dt, mu, p.starter,
-                                                                             p.mlp, p.tol_dt);
-                    fl = d.flags;
-                    evals += d.evals;
-                    if constexpr (LEARNED) nets += d.net;
-                    wide += d.wide;
+                    GFun g;
+                    double mu_r;
+                    if constexpr (!LEARNED) {
+                        if (p.starter != STARTER_CLASSIC && q3 < 0.5f * MEDIUM_DRIFT_TAU2) {
+                            ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
+                            tier = small_drift<true>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt,
+                                                     p.sdt, sd);
+                        }
+                    }
+                    if (tier == DRIFT_MEDIUM) {
+                        mu_r = mu * rinv[k];
+                        medium_gfuns(sd, p.dt * rinv[k], g.g1, g.g2, g.g3);
+                        evals++;
+                    } else {
+                        const DriftInvariants q =
+                            drift_invariants(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], p.dt, mu);
+                        const DriftResult d = kepler_solve<LEARNED, NET_ROWS, NET_QU>(g, rinv[k], q, p.dt, mu, p.starter,
+                                                                                      p.mlp, p.tol_dt);
+                        mu_r = q.mu_r;
+                        fl = d.flags;
+                        evals += d.evals;
+                        if constexpr (LEARNED) nets += d.net;
+                        wide += d.wide;
+                    }
+                    drift_apply(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], g, mu_r, p.dt, mu);
                     ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
                     f2[k] = ff_split_fast(r2[k]);
                     fri[k] = ff_split_fast(rinv[k]);

@@ -54,6 +54,22 @@ def test_block_of_drifts(lo, hi, steps, kick):
         assert err.max() < tol, (err.max(), tol)
 
 
+@pytest.mark.parametrize("steps", [1, 2])
+def test_block_of_drifts_at_the_medium_bound(steps):
+    # tau^2 around 1e-2, where the float-float solution gives way to the general one
+    rng = np.random.default_rng(15)
+    rv = states(np.exp(rng.uniform(np.log(0.8e-2), np.log(1.2e-2), N)), rng.uniform(0, 0.6, N), 16)
+    got, _ = block(rv, steps, G.KICK_FLOAT_FLOAT)
+    want = rv.astype(np.longdouble)
+    for _ in range(steps):
+        want = np.concatenate(drift_long_double(want, DT, MU), 1)
+    tol = 1.2e-15 * steps * (1 + 4 * np.sqrt(1.2e-2) * steps)      # as above
+    for s in (slice(0, 3), slice(3, 6)):
+        d = (got[:, s] - want[:, s]).astype(np.float64)
+        err = np.linalg.norm(d, axis=1) / np.linalg.norm(want[:, s].astype(np.float64), axis=1)
+        assert err.max() < tol, (err.max(), tol)
+
+
 def test_a_particles_path_is_its_own():
     rng = np.random.default_rng(13)
     rv = states(np.exp(rng.uniform(np.log(1e-4), np.log(5e-3), N)), np.full(N, 0.05), 14)

@@ -164,3 +164,59 @@ def test_drift_leaves_what_is_outside_its_domain(lib):
         ok = np.zeros(n, np.int32)
         lib.drift(n, C.c_double(DT), C.c_double(MU), ptr(rv), ptr(ok))
         assert not ok.any() and np.array_equal(rv, before, equal_nan=True)
+
+
+def gfuns_long_double(rv, dt, mu):
+    r, v = rv[:, :3].astype(LD), rv[:, 3:].astype(LD)
+    dt, mu = LD(dt), LD(mu)
+    r0 = np.sqrt((r * r).sum(1))
+    u = (r * v).sum(1)
+    al = 2 * mu / r0 - (v * v).sum(1)
+    s = dt / r0
+    for _ in range(10):
+        x = al * s * s
+        c2, c3 = LD(0), LD(0)
+        f2, f3 = LD(1) / 2, LD(1) / 6
+        for k in range(12):
+            c2, c3 = c2 + f2, c3 + f3
+            f2, f3 = -f2 * x / ((2 * k + 3) * (2 * k + 4)), -f3 * x / ((2 * k + 4) * (2 * k + 5))
+        g2, g3 = s * s * c2, s * s * s * c3
+        g0, g1 = 1 - al * g2, s - al * g3
+        s = s - (r0 * g1 + u * g2 + mu * g3 - dt) / (r0 * g0 + u * g1 + mu * g2)
+    return g1, g2, g3
+
+
+@pytest.mark.parametrize("lo,hi", [(1.0001e-3, 2e-3), (2e-3, 5e-3), (5e-3, 0.9999e-2)])
+@pytest.mark.parametrize("kind", ["spread", "circular", "retrograde", "eccentric"])
+def test_medium_solution_against_long_double(lib, lo, hi, kind):
+    n = 4000
+    rng = np.random.default_rng(17)
+    e = {"circular": np.zeros(n), "eccentric": rng.uniform(0.9, 0.99, n)}.get(kind, rng.uniform(0, 0.9, n))
+    rv = states(np.exp(rng.uniform(np.log(lo), np.log(hi), n)), e, 18, -1.0 if kind == "retrograde" else 1.0)
+    tier, g = np.zeros(n, np.int32), np.zeros((n, 3))
+    lib.gfuns_medium(n, C.c_double(DT), C.c_double(MU), ptr(rv), ptr(tier), ptr(g))
+    assert (tier == 2).all()
+    want = gfuns_long_double(rv, DT, MU)
+    r0 = np.linalg.norm(rv[:, :3], axis=1)
+    v0 = np.linalg.norm(rv[:, 3:], axis=1)
+    # what the G-functions carry into the state: mu G2 / r0 into r, mu G3 into the
+    # time step, mu G1 / r0^2 and mu G2 / r0 into v; each may add a quarter of the
+    # state's own FP64 rounding: 2^-55 of |r0| and 2^-53 of the velocity's scale
+    vs = np.maximum(v0, np.sqrt(MU / r0))
+    d1, d2, d3 = (np.abs(g[:, k] - want[k]) for k in range(3))
+    assert np.all(MU * d2 / r0 <= 2.0 ** -55)
+    assert np.all(MU * d3 * v0 / r0 <= 2.0 ** -55)
+    assert np.all(MU * d1 / r0 <= 2.0 ** -53 * vs)
+    assert np.all(MU * d2 / r0 * v0 <= 2.0 ** -53 * vs)
+
+
+def test_medium_solution_leaves_the_rest(lib):
+    n = 500
+    e = np.full(n, 0.3)
+    below, above = states(np.full(n, 0.999e-3), e, 21), states(np.full(n, 1.001e-2), e, 22)
+    fast = states(np.full(n, 5e-3), e, 23)
+    fast[:, 3:] *= 1.5 * np.sqrt(2 * MU / np.linalg.norm(fast[:, :3], axis=1) / (fast[:, 3:] ** 2).sum(1))[:, None]
+    for rv, want in ((below, 1), (above, 0), (fast, 0)):
+        tier, g = np.full(n, -1, np.int32), np.zeros((n, 3))
+        lib.gfuns_medium(n, C.c_double(DT), C.c_double(MU), ptr(rv), ptr(tier), ptr(g))
+        assert (tier == want).all() and not g.any()
