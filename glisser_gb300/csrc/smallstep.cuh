@@ -274,14 +274,15 @@ __device__ __forceinline__ float kepler_residual(ff X, ff Y, float w, ff q2, ff 
 // float-float velocity, but Kepler's equation can still be solved here: the FP64
 // G-functions are T (1 - e), (T^2/2)(1 + q2), (T^3/6)(1 + q3) with T = dt / r0, and
 // e, q2, q3 of 0.2 at most.  It spares the general solution's invariants, FP64
-// residual and Stumpff series (about 30 FP64 instructions).  An instance of its own,
-// and not in the kernel of the learned starter: with one code for both tiers (the
-// shared half not repeated) the scattered disk took 6.19 instead of 6.47 ms, but
-// its registers cost the planet crossers 2 % and the ensembles 5 %.  The line at 1e-2:
-// e, q2 and q3 at 2^-46 then change r by 2^-55 and v by 2^-53 at most, and the series
-// end below 2^-46.  300,000 scattered-disk particles x 180 steps, 0.9 % of their drifts
-// here and 0.1 % beyond, but spread over a quarter of the warps: 7.19 -> 6.47 ms,
-// error against long double 3.1e-15 before and after.
+// residual and Stumpff series (about 30 FP64 instructions).  An instance of its own:
+// with one code for both tiers (the shared half not repeated) the scattered disk
+// took 6.19 instead of 6.47 ms, but its registers cost the planet crossers 2 % and
+// the ensembles 5 %.  The line at 1e-2: e, q2 and q3 at 2^-46 then change
+// r by 2^-55 and v by 2^-53 at most, and the series end below 2^-46.  300,000
+// scattered-disk particles x 256 steps, 0.9 % of their drifts here and 0.1 % beyond,
+// but spread over a quarter of the warps: 7.19 -> 6.47 ms, error against long double
+// 3.1e-15 before and after; 1e6 particles x 64 steps with the learned starter
+// 5.94 -> 5.21 ms.
 template <bool MEDIUM>
 __device__ __forceinline__ int small_drift(ff rx, ff ry, ff rz, ff vx, ff vy, ff vz, ff r2, ff rinv, ff muh, ff mudt,
                                            const SmallStepDt& c, SmallDrift& d)

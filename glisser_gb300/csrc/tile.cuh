@@ -368,12 +368,9 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                     }
                     GFun g;
                     double mu_r;
-                    if constexpr (!LEARNED) {
-                        if (p.starter != STARTER_CLASSIC && q3 < 0.5f * MEDIUM_DRIFT_TAU2) {
-                            ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
-                            tier = small_drift<true>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt,
-                                                     p.sdt, sd);
-                        }
+                    if (p.starter != STARTER_CLASSIC && q3 < 0.5f * MEDIUM_DRIFT_TAU2) {
+                        ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
+                        tier = small_drift<true>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
                     }
                     if (tier == DRIFT_MEDIUM) {
                         mu_r = mu * rinv[k];
