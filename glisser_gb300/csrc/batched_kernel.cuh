@@ -11,19 +11,18 @@ namespace {
 using namespace tile;
 
 // Resident threads per SM the ensemble kernel's registers are sized for; a
-// build-time tuning knob.  The plain-starter kernel is latency-bound (FP64
-// pipe ~65 % busy, issue ~57 % at 5 CTAs of 128), so it is sized for 8 CTAs
-// of 128 per SM (64 registers, ~100 bytes of spills; 64-step planet-log
-// chunks fit 8 CTAs' shared memory): 6 % faster than 5 CTAs at 93
-// registers, and ahead of 6, 7 and 9 CTAs.  The learned-starter kernel is
-// sized the same: on ensembles whose every drift runs the network it
-// measured 1.6 % faster at 8 CTAs (64 registers, its network's activations
-// and spills in local memory) than at 4 (96 registers).
+// build-time tuning knob.  The kernel is bound by issue, and spills are
+// instructions: 768 (80 registers, 6 CTAs of 128, 32 bytes of spill stores and loads)
+// run the 256 giants systems' 512-step block in 34.8 ms, 1,024 (64 registers, 360
+// bytes) in 37.2, 896 in 35.7 to 36.7, 640 in 36.2, 512 in 35.9.  Systems whose every drift is general
+// (close-eccentric, bound by the FP64 pipe) run 1.5 % slower at 768 than at 1,024.
+// The learned-starter kernel, which a block takes only when some drifts are wide,
+// stays at 1,024: 2 % faster than at 768 where every drift runs the network.
 #ifndef GLISSER_BATCHED_THREADS_PER_SM
-#define GLISSER_BATCHED_THREADS_PER_SM 1024
+#define GLISSER_BATCHED_THREADS_PER_SM 768
 #endif
 #ifndef GLISSER_BATCHED_THREADS_PER_SM_LEARNED
-#define GLISSER_BATCHED_THREADS_PER_SM_LEARNED GLISSER_BATCHED_THREADS_PER_SM
+#define GLISSER_BATCHED_THREADS_PER_SM_LEARNED 1024
 #endif
 
 // Persistent kernel over (system, tile) work items.  The learned starter
