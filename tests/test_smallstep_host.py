@@ -220,3 +220,23 @@ def test_medium_solution_leaves_the_rest(lib):
         tier, g = np.full(n, -1, np.int32), np.zeros((n, 3))
         lib.gfuns_medium(n, C.c_double(DT), C.c_double(MU), ptr(rv), ptr(tier), ptr(g))
         assert (tier == want).all() and not g.any()
+
+
+@pytest.mark.parametrize("e_max", [0.0, 0.6, 0.99])
+def test_drift_far_out_against_long_double(lib, e_max):
+    # the lower end of the domain, tau^2 down to 2^-33: every correction is below
+    # tau^2, so one FP64 rounding a component and 2^-40 of the correction remain
+    n = 4000
+    rng = np.random.default_rng(31)
+    rv = states(np.exp(rng.uniform(np.log(1.2e-10), np.log(1e-8), n)), rng.uniform(0, e_max, n), 32)
+    want_r, want_v = drift_long_double(rv, DT, MU)
+    v0, r0 = np.linalg.norm(rv[:, 3:], axis=1), np.linalg.norm(rv[:, :3], axis=1)
+    ok = np.zeros(n, np.int32)
+    lib.drift(n, C.c_double(DT), C.c_double(MU), ptr(rv), ptr(ok))
+    assert ok.mean() > 0.99
+    k = ok == 1
+    er = np.sqrt(((rv[:, :3] - want_r) ** 2).sum(1)) / r0
+    ev = np.sqrt(((rv[:, 3:] - want_v) ** 2).sum(1)) / v0
+    kick = np.sqrt(MU / r0 ** 3) * DT * np.sqrt(MU / r0) / v0
+    assert np.all(er[k] <= 2.0 ** -53 * np.sqrt(3) + 1e-8 * 2.0 ** -40)
+    assert np.all(ev[k] <= 2.0 ** -53 * np.sqrt(3) + (2.0 ** -45 * kick)[k])
