@@ -20,11 +20,10 @@ using namespace tile;
 
 // The learned-starter kernel runs the network per lane, inline, only where
 // the series starter is outside its domain.  Sized for 14 CTAs of 64 (72
-// registers): the network's registers cost less there than its spills at 16
-// (64 registers), 3.41 against 4.43 ms for a 128-step block of 100,000
-// close-eccentric particles, 14.55 against 14.62 ms for 64 steps of 1e6, and
-// 5.93 against 5.78 ms on 1e6 scattered-disk particles, where 0.1 % of drifts
-// take the network.  The network's shape (mlp_forward: four rows of the hidden
+// registers; a second instance, below, for 16): the network's registers cost less
+// there than its spills at 16 (64 registers): 14.46 against 14.66 ms for 64 steps of
+// 1e6 close-eccentric particles; 5.31 against 5.15 ms on 1e6 scattered-disk
+// particles, where 0.1 % of drifts take the network.  The network's shape (mlp_forward: four rows of the hidden
 // layer per pass, two activation reads in flight) was chosen for a register
 // budget.
 #ifndef GLISSER_TB_MIN_BLOCKS_LEARNED
@@ -41,8 +40,8 @@ constexpr int TB_NET_QU = 2;
 #define GLISSER_TB_PPT 1
 #endif
 
-template <int NP, bool LEARNED, bool KICK64>
-__global__ void __launch_bounds__(BLOCK_THREADS, LEARNED ? GLISSER_TB_MIN_BLOCKS_LEARNED : GLISSER_TB_MIN_BLOCKS)
+template <int NP, bool LEARNED, bool KICK64, int CTAS_PER_SM>
+__global__ void __launch_bounds__(BLOCK_THREADS, CTAS_PER_SM)
     timeblock_kernel(const Common p, const double* log, const double* m, const double* rh, const uint32_t* pid,
                      uint32_t n)
 {
@@ -58,16 +57,44 @@ __global__ void __launch_bounds__(BLOCK_THREADS, LEARNED ? GLISSER_TB_MIN_BLOCKS
         p, log, first, min((uint32_t)(BLOCK_THREADS * PPT), n - first), stage, sh, phase);
 }
 
+// The learned kernel's second instance, sized for the plain kernel's CTAs per SM,
+// runs a grid that it takes in fewer waves: a wave of a few CTAs lasts as long as
+// their serial chain.  100,000 close-eccentric particles x 128 steps (one wave of
+// either) 3.40 ms with 14 CTAs and 4.44 with 16, 135,000 4.12 and 4.49, 140,000 (two
+// waves of 14) 5.34 and 4.58, 150,000 5.70 and 4.83.
+inline bool learned_saves_a_wave(uint32_t grid, uint32_t sms)
+{
+    const uint32_t lean = sms * GLISSER_TB_MIN_BLOCKS_LEARNED, full = sms * GLISSER_TB_MIN_BLOCKS;
+    return (grid + full - 1) / full < (grid + lean - 1) / lean;
+}
+
+template <int NP, bool LEARNED, bool KICK64, int CTAS_PER_SM>
+cudaError_t launch_sized(const Common& p, const glisser_planet_block* pl, uint32_t n, uint32_t grid, size_t smem,
+                         cudaStream_t stream)
+{
+    auto kern = timeblock_kernel<NP, LEARNED, KICK64, CTAS_PER_SM>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, BLOCK_THREADS, smem, stream>>>(p, pl->log, pl->m, pl->rh, pl->id, n);
+    return cudaGetLastError();
+}
+
 template <int NP, bool LEARNED, bool KICK64>
 cudaError_t launch_np(const Common& p, const glisser_planet_block* pl, uint32_t n, size_t smem, cudaStream_t stream)
 {
-    auto kern = timeblock_kernel<NP, LEARNED, KICK64>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     const uint32_t per_cta = (uint32_t)BLOCK_THREADS * (LEARNED ? 1u : (uint32_t)GLISSER_TB_PPT);
     const uint32_t grid = (n + per_cta - 1) / per_cta;
-    kern<<<grid, BLOCK_THREADS, smem, stream>>>(p, pl->log, pl->m, pl->rh, pl->id, n);
-    return cudaGetLastError();
+    if constexpr (LEARNED) {
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (learned_saves_a_wave(grid, (uint32_t)sms))
+            return launch_sized<NP, LEARNED, KICK64, GLISSER_TB_MIN_BLOCKS>(p, pl, n, grid, smem, stream);
+        return launch_sized<NP, LEARNED, KICK64, GLISSER_TB_MIN_BLOCKS_LEARNED>(p, pl, n, grid, smem, stream);
+    } else {
+        return launch_sized<NP, LEARNED, KICK64, GLISSER_TB_MIN_BLOCKS>(p, pl, n, grid, smem, stream);
+    }
 }
 
 // Dispatch over the planet count for one kernel variant.
