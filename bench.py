@@ -55,20 +55,21 @@ ENSEMBLE_WORKLOAD = ("ensembles: 256 systems (Sun + 4 giants, masses x U(0.9,1.1
 
 # Executed FP64 thread-instructions per particle-step counted by ncu
 # (smsp__sass_thread_inst_executed_op_d{add,fma,mul}_pred_on.sum over one
-# launch, divided by the launch's particle-steps) and the FP64 pipe's busy
-# share (sm__pipe_fp64_cycles_active, pct of peak sustained active), for the
+# launch, divided by the launch's particle-steps), the FP64 pipe's busy share
+# (sm__pipe_fp64_cycles_active, pct of peak sustained active) and that of the
+# issue slots (smsp__issue_active), which bound these kernels, for the
 # kernels whose rooflines the bench reports; the captures and their commands
 # are summarised under profiles/.
 FP64_COUNTS = {
-    "batched_kernel<4,128,1,series>": {"dadd": 1.0, "dfma": 26.0, "dmul": 17.0, "pipe_busy": 0.776,
+    "batched_kernel<4,128,1,series>": {"dadd": 6.0, "dfma": 5.1, "dmul": 1.2, "pipe_busy": 0.491, "issue_busy": 0.857,
                                        "profile": "profiles/batched_kernel_ensembles.md"},
-    "timeblock_kernel<4>": {"dadd": 1.0, "dfma": 26.0, "dmul": 17.0, "pipe_busy": 0.709,
+    "timeblock_kernel<4>": {"dadd": 6.0, "dfma": 5.0, "dmul": 1.3, "pipe_busy": 0.446, "issue_busy": 0.781,
                             "profile": "profiles/timeblock_kernel_plain-giants.md"},
 }
 # DRAM bytes per particle per block of the batched kernel (ncu dram__bytes_read
-# + dram__bytes_write, 153.2 + 78.8 MB, on a capture of one block of a quarter
-# of the headline workload: 1,537,972 particles, T = 1024)
-DRAM_BYTES_PER_PARTICLE_BLOCK = 150.8
+# + dram__bytes_write, 113.4 + 60.9 MB, on a capture of one block of 256 systems
+# of the same kind with 1,500,000 particles)
+DRAM_BYTES_PER_PARTICLE_BLOCK = 116.2
 
 
 def alg_flops_per_particle_step(n_planets, k_ref=5):
@@ -96,7 +97,8 @@ def executed_fp64(kernel, rate, peak_tf):
     return {"kernel": kernel, "counts_from": key,
             "instructions_per_particle_step": round(c["dadd"] + c["dmul"] + c["dfma"], 1),
             "flops_per_particle_step": flops, "achieved": tf, "peak": peak_tf, "unit": "TFLOP/s",
-            "frac": tf / peak_tf if peak_tf else None, "fp64_pipe_busy": c["pipe_busy"], "source": c["profile"]}
+            "frac": tf / peak_tf if peak_tf else None, "fp64_pipe_busy": c["pipe_busy"],
+            "issue_busy": c["issue_busy"], "source": c["profile"]}
 
 
 def config_text(tbsize, dt, outer=300.0, extra=""):
@@ -507,7 +509,8 @@ def run_headline(G, args, rank, world, path, barrier, peak_tf, local):
                        "FP64 figure",
         "achieved_is": "executed FP64 flops (ncu DADD + DMUL + 2 DFMA per particle-step of this build) x the "
                        "kernel's particle-step rate from CUDA events around each launch",
-        "fp64_pipe_busy": ex["fp64_pipe_busy"] if ex else None, "executed": ex,
+        "fp64_pipe_busy": ex["fp64_pipe_busy"] if ex else None,
+        "issue_busy": ex["issue_busy"] if ex else None, "executed": ex,
         "reference_formulation": {"flops_per_particle_step": F, "achieved": kernel_rate * F / 1e12,
                                   "frac": kernel_rate * F / 1e12 / peak_tf if peak_tf else None,
                                   "note": "the reference's algorithmic flops (five Newton passes with sin/cos "

@@ -5,7 +5,7 @@
 //   device, planet stream: the next block's planet WH for every system (one
 //           warp per system, planets_dev.cu) writing the planet logs and
 //           encounter radii the next block stages, launched just before this
-//           block's kernel so its few CTAs take SMs first;
+//           block's kernel so its one-warp CTAs are resident first;
 //   host  : the (system, tile) work items of the tiles that still hold alive
 //           particles;
 //   device: one CUDA graph per staging parity, captured once: upload of the
@@ -589,8 +589,8 @@ double Ensemble::step(double* gpu_ms)
     for (auto a : alive_) before_alive += a;
     if (device_planets_) {
         // this block waits for its planet logs; the next block's planets are
-        // launched before this block's kernel so that their few CTAs take SMs
-        // first and run alongside the persistent kernel
+        // launched before this block's kernel so that their one-warp CTAs are
+        // resident first and run alongside the persistent kernel
         ck(cudaStreamWaitEvent(d.stream, d.planets_done, 0), "wait planets");
         planets_device(par ^ 1);
     }

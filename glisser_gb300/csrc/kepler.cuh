@@ -1,4 +1,6 @@
-// Universal-variable Kepler drift for the particle time-block kernel.
+// Universal-variable Kepler drift for the particle time-block kernel: the general
+// drift, for the steps that smallstep.cuh leaves (there the time-block kernels solve
+// and apply a drift on the FP32 pipe), for the classic starter and for single drifts.
 //
 // Solves  f(s) = r0*G1(s) + u*G2(s) + mu*G3(s) - dt = 0  for the universal
 // anomaly s, with G_k(s) = s^k c_k(alpha s^2) the Stumpff-scaled G-functions

@@ -89,8 +89,7 @@ __device__ __forceinline__ float mlp_sigmoid(float a) { return __fdividef(1.0f, 
 // is a fraction of a row-at-a-time loop's; QU activation reads per row group
 // are in flight at once.  Each row's sum keeps the order of the training
 // kernels' forward pass, so neither changes the result, only the registers
-// and the latency: the single-system learned kernel, whose register budget
-// has room, unrolls further than the ensemble kernel.
+// and the latency.
 constexpr int MLP_ROWS = 4;
 
 template <int ROWS = MLP_ROWS, int QU = 1>

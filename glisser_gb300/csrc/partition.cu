@@ -229,7 +229,8 @@ int launch_partition(const glisser_particles* in, const glisser_particles* out, 
 // file-scope device array instead.
 //
 // NOALLOC_MAX_PARTICLES bounds n: room for 2 counts per 256-particle tile (the
-// ranges use fewer), 256 KiB in all, resident on every GPU that loads the library until the process exits.
+// ranges use fewer), 256 KiB in all, resident on every GPU that loads the library
+// until the process exits.
 // Every call shares that array and leaves the last call's counts in it.  No
 // entry needs clearing before a call (count_kernel writes every range's counts
 // before scatter_kernel reads them), but two calls whose work overlaps on the

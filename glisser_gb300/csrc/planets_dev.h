@@ -26,7 +26,8 @@ constexpr uint32_t PLANET_WH_MAX_NPL = 32;
 // planet-log records (per step: h0, then planets 1..npl-1) at
 // log + s * log_stride, and the encounter radii of the block's start state
 // (cull radius for the Sun; rh_factor x Hill radius at pericentre for the
-// planets when |rh_factor| > 1e-6) at rh + s * npl.  One warp per system.
+// planets when |rh_factor| > 1e-6) at rh + s * npl.  One warp per system: a lane
+// per vector component up to five planets, a lane per planet above.
 cudaError_t launch_planet_wh(const PlanetSysDev& ps, uint32_t systems, uint32_t npl, uint32_t len, double dt,
                              double cull_radius, double rh_factor, double* log, size_t log_stride, double* rh,
                              cudaStream_t stream);

@@ -8,8 +8,9 @@
 // 8-byte-per-lane access.  The planet log (per step: h0, then the planet
 // positions) is staged into shared memory in chunks of `chunk` steps by bulk
 // TMA copies (cp.async.bulk ... mbarrier::complete_tx), double buffered, and
-// read from there as warp-wide broadcasts.  The drift is the universal-
-// variable solver of kepler.cuh.  Flag semantics follow the reference kernel
+// read from there as warp-wide broadcasts.  The drift is the
+// float-float one of smallstep.cuh for small steps, else the universal-variable
+// solver of kepler.cuh.  Flag semantics follow the reference kernel
 // (src/wh.cu:132-176): the first planet inside its radius marks the particle
 // with (planet id << 8) | 0x01, the Sun's radius overrides with 0x01 and the
 // outer limit with 0x02, and a flagged particle stops for the rest of the
