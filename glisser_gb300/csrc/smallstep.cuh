@@ -106,17 +106,24 @@ __device__ __forceinline__ ff ff_sqr3(ff x, ff y, ff z) { return ff_sum3(ff_sqr_
 // turns their branches into predicated instructions that every step issues
 // (ff_widen's FP64 conversions and addition, so issued, made the crossers'
 // block 1.9x longer).
-static __device__ __noinline__ ff ff_split_rare(double d) { return ff_split(d); }
+static __device__ __noinline__ ff ff_split_rare(double d)
+{
+    if (d != d) return { __int_as_float(0x7fc00000), __int_as_float(0x7fc00000) };
+    if (fabs(d) >= 0x1p128) return { f32_trunc(d), 0.0f };      // infinity
+    return ff_split(d);
+}
 static __device__ __noinline__ double ff_widen_rare(float hi, float lo) { return (double)hi + (double)lo; }
 
 // A double as a float-float on the integer and FP32 pipes: hi = d rounded to
 // 24 significant bits, lo = the (signed) rest rounded to 24: |d - hi - lo| <
-// 2^-49 |d|, for |d| < 2^127.  ff_split counts leading zeros to place lo; here
-// the conversion instruction does.  Zero and |d| < 2^-70 (where lo's unit would
-// leave the float range) are rare: they take ff_split.
+// 2^-49 |d|, for 2^-70 <= |d| < 2^127.  ff_split counts leading zeros to place
+// lo; here the conversion instruction does.  Zero and |d| < 2^-70 (where lo's unit
+// would leave the float range), |d| >= 2^127, the infinities and NaN (whose
+// exponents would wrap into a float's) are rare: they take ff_split_rare.
 __device__ __forceinline__ bool split_is_rare(double d)
 {
-    return ((unsigned)__double2hiint(d) & 0x7fffffffu) < ((1023u - 70u) << 20);
+    // both ends in one unsigned comparison, the sign shifted out
+    return 2u * (unsigned)__double2hiint(d) - ((1023u - 70u) << 21) >= (127u + 70u) << 21;
 }
 
 __device__ __forceinline__ ff split_common(double d)
@@ -155,12 +162,12 @@ __device__ __forceinline__ void ff_split3(double x, double y, double z, ff& fx, 
 // hi + lo as a double on the integer and FP32 pipes, to ~2^-47 of it (lo
 // enters in units of 2^-46 of hi's binade), for a renormalised pair: hi widened
 // exactly, lo's multiple of the unit added to the magnitude bits.  hi a power
-// of two (the sum may fall into the binade below, whose unit is another), zero
-// or below 2^-76 is rare: it takes the FP64 addition.
+// of two (the sum may fall into the binade below, whose unit is another), zero,
+// below 2^-76, infinite or NaN is rare: it takes the FP64 addition.
 __device__ __forceinline__ bool widen_is_rare(ff x)
 {
     const unsigned b = __float_as_uint(x.hi);
-    return (b & 0x007fffffu) == 0u || fabsf(x.hi) < 0x1p-76f;
+    return (b & 0x007fffffu) == 0u || !(fabsf(x.hi) >= 0x1p-76f);
 }
 
 __device__ __forceinline__ double widen_common(ff x)
@@ -273,7 +280,9 @@ __device__ __forceinline__ float kepler_residual(ff X, ff Y, float w, ff q2, ff 
 // Solves one drift from the float-float split of its state, of r0^2 and 1/r0
 // (muh = mu dt^2 / 2, mudt = mu dt).  DRIFT_GENERAL (nothing solved) for tau^2 at or
 // above the tier's bound, a state not bound beyond the energy's rounding, or a
-// value outside the range that float-float covers (a NaN in 1/r0 says so).  The
+// value outside the range that float-float covers (run_tile puts a NaN in 1/r0
+// where |r|^2 leaves it; a NaN or an infinity in any input leaves tau^2 or the
+// energy's A NaN or -infinity, which no comparison below accepts).  The
 // decision is each particle's own, so that its path does not depend on the
 // particles that share its warp.
 //
