@@ -563,9 +563,9 @@ __device__ __forceinline__ void load_planet_constants(const Common& p, CtaShared
         q.near2 = m[j] == 0.0 || (am > KICK_MDT_MIN && am < KICK_MDT_MAX) ? near : __int_as_float(0x7f800000);
         sh.pk[j] = q;
         if (j == 0) {
-            const double muh = 0.5 * m[0] * p.dt * p.dt;
-            sh.muh = ff_split_fast(muh);
-            sh.mudt = ff_split(-mdt);
+            const SmallStepMu c = small_step_mu(m[0], p.dt);
+            sh.muh = c.muh;
+            sh.mudt = c.mudt;
             // outside the range the constant's products cover, NaN: the general drift runs
             if (!(sh.muh.hi > 0x1p-40f && sh.muh.hi < 0x1p30f)) sh.muh.hi = __int_as_float(0x7fc00000);
             sh.muh.hi *= p.dt_range;
