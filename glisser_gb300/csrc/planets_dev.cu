@@ -89,9 +89,12 @@ __device__ int kepler_drift_planet(double mu, double dt, double& rx, double& ry,
 // fourth-order reversion and three FP32 Newton steps leave s within ~1e-7, one
 // FP64 evaluation of the G-functions (|x| < 0.3: stumpff_small's next term is
 // 2e-17) with the second-order Newton correction folded in does the rest.
-// Wider steps, other orbits and values outside a float's range take
-// kepler_drift_planet, whose refusals stay.
-__device__ __forceinline__ bool jacobi_start(float t, float u, float rinv, float alpha, float mu_r, float& w)
+// Wider steps, other orbits and values outside a float's range (mu itself, which
+// the correction's second-order term takes in FP32: G Msun in cm^3/yr^2 is above
+// it) take kepler_drift_planet, whose refusals stay.
+constexpr float JACOBI_MU_MAX = 1e37f;       // alpha r0, below 2 mu, stays a float too
+
+__device__ __forceinline__ bool jacobi_start(float t, float u, float rinv, float alpha, float mu_r, float mu, float& w)
 {
     const float tau2 = t * t * mu_r;
     const float X = 0.5f * u * rinv * t, A = alpha * t * t, Y = (tau2 - A) * (1.0f / 6.0f);
@@ -105,7 +108,7 @@ __device__ __forceinline__ bool jacobi_start(float t, float u, float rinv, float
         const float Rp = fmaf(2.0f * X * s, fmaf(x * (-1.0f / 6.0f), c3, 1.0f), fmaf(3.0f * Y * s2, c2, 1.0f));
         w -= __fdividef(R, Rp);
     }
-    return A > 1e-12f && A < 0.25f && tau2 < 0.25f && fabsf(X) < 0.15f;
+    return A > 1e-12f && A < 0.25f && tau2 < 0.25f && fabsf(X) < 0.15f && mu < JACOBI_MU_MAX;
 }
 
 // The Newton correction ds of s from f, f' and G0, G1: h = f / f' from the FP32
@@ -129,9 +132,9 @@ __device__ __forceinline__ int kepler_drift_jacobi(double mu, double dt, double&
     const double rinv = rsqrt_fast(r2);
     const double r0 = r2 * rinv, u = fma(rx, vx, fma(ry, vy, rz * vz)), mu_r = mu * rinv, T = dt * rinv;
     const double alpha = fma(2.0, mu_r, -fma(vx, vx, fma(vy, vy, vz * vz)));
-    const float uf = f32_trunc(u), af = f32_trunc(alpha);
+    const float uf = f32_trunc(u), af = f32_trunc(alpha), muf = f32_trunc(mu);
     float w;
-    if (!jacobi_start(f32_trunc(T), uf, f32_trunc(rinv), af, f32_trunc(mu_r), w))
+    if (!jacobi_start(f32_trunc(T), uf, f32_trunc(rinv), af, f32_trunc(mu_r), muf, w))
         return kepler_drift_planet(mu, dt, rx, ry, rz, vx, vy, vz);
     const double s = fma(T, f64_of_f32(w), T), s2 = s * s, x = alpha * s2;
     double c2, c3;
@@ -139,7 +142,7 @@ __device__ __forceinline__ int kepler_drift_jacobi(double mu, double dt, double&
     const double g2 = s2 * c2, g3 = s * (s2 * c3), g1 = fma(-alpha, g3, s), g0 = fma(-alpha, g2, 1.0);
     const double f = fma(r0, g1, fma(u, g2, fma(mu, g3, -dt)));
     const double fp = fma(r0, g0, fma(u, g1, mu * g2));
-    const double ds = jacobi_correction(f, fp, f32_trunc(r0), uf, f32_trunc(mu), af, g0, g1), hd = 0.5 * ds;
+    const double ds = jacobi_correction(f, fp, f32_trunc(r0), uf, muf, af, g0, g1), hd = 0.5 * ds;
     const double n3 = fma(ds, fma(hd, g1, g2), g3), n2 = fma(ds, fma(hd, g0, g1), g2);
     const double n1 = fma(ds, fma(-alpha * hd, g1, g0), g1);
     const double ff = fma(-mu_r, n2, 1.0), gg = fma(-mu, n3, dt);
@@ -424,7 +427,7 @@ __global__ void __launch_bounds__(32)
             const double alpha = fma(2.0, mu_r, -v2);
             const float uf = f32_trunc(u), af = f32_trunc(alpha);
             float wf;
-            const bool inside = jacobi_start(f32_trunc(T), uf, f32_trunc(rinv), af, f32_trunc(mu_r), wf);
+            const bool inside = jacobi_start(f32_trunc(T), uf, f32_trunc(rinv), af, f32_trunc(mu_r), muf, wf);
             const double sv = fma(T, f64_of_f32(wf), T), s2 = sv * sv, x = alpha * s2;
             double h = fma(x, k6, k5);
             h = fma(x, h, k4);
