@@ -87,8 +87,10 @@ __device__ int kepler_drift_planet(double mu, double dt, double& rx, double& ry,
 // anomaly iteration always converges too).  Kepler's equation in the
 // dimensionless form R(w) = 0 of smallstep.cuh, s = (dt / r0)(1 + w): its
 // fourth-order reversion and three FP32 Newton steps leave s within ~1e-7, one
-// FP64 evaluation of the G-functions (|x| < 0.3: stumpff_small's next term is
-// 2e-17) with the second-order Newton correction folded in does the rest.
+// FP64 evaluation of the G-functions (|x| < 0.4, for inbound orbits at the bounds:
+// stumpff_small's next term is 1.4e-16 of c2, which mu G2 / r0 < 0.13 carries into
+// the position as 2e-17) with the second-order Newton correction folded in does the
+// rest.
 // Wider steps, other orbits and values outside a float's range (mu itself, which
 // the correction's second-order term takes in FP32: G Msun in cm^3/yr^2 is above
 // it) take kepler_drift_planet, whose refusals stay.
