@@ -34,6 +34,7 @@
 #include "ensemble.h"
 #include "parallel.h"
 #include "executor.h"
+#include "hostcopy.h"
 #include "mlp_train.h"
 #include "planets_dev.h"
 #include "timeblock.cuh"
@@ -432,10 +433,10 @@ void Ensemble::init()
     q += cap * sizeof(uint32_t);
     d.pa.flags = reinterpret_cast<uint16_t*>(q);
     for (int k = 0; k < 9; k++)
-        ck(cudaMemcpy(*dbl[k], col.data() + k * total, total * sizeof(double), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(d.pa.flags, flags_.data(), total * sizeof(uint16_t), cudaMemcpyHostToDevice), "upload flags");
-    ck(cudaMemcpy(d.pa.id, ids_.data(), total * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload ids");
-    ck(cudaMemset(d.pa.deathtime_index, 0, total * sizeof(uint32_t)), "memset");
+        ck(copy_to_device(*dbl[k], col.data() + k * total, total * sizeof(double)), "upload");
+    ck(copy_to_device(d.pa.flags, flags_.data(), total * sizeof(uint16_t)), "upload flags");
+    ck(copy_to_device(d.pa.id, ids_.data(), total * sizeof(uint32_t)), "upload ids");
+    ck(clear_on_device(d.pa.deathtime_index, total * sizeof(uint32_t)), "memset");
 
     // planet blocks: per system stride rounded to 16 bytes
     uint32_t recs = (len_ + 1u) & ~1u;
@@ -508,11 +509,11 @@ void Ensemble::init()
                 }
             }
         }
-        ck(cudaMemcpy(d.pl.rx, h.data(), 14 * cnt * sizeof(double), cudaMemcpyHostToDevice), "upload planets");
-        ck(cudaMemset(d.pl.status, 0, S * sizeof(uint32_t)), "memset");
+        ck(copy_to_device(d.pl.rx, h.data(), 14 * cnt * sizeof(double)), "upload planets");
+        ck(clear_on_device(d.pl.status, S * sizeof(uint32_t)), "memset");
         for (int b = 0; b < 2; b++) {
-            ck(cudaMemcpy(d.d_m[b], d.h_m[b], cnt * sizeof(double), cudaMemcpyHostToDevice), "upload m");
-            ck(cudaMemcpy(d.d_id[b], d.h_id[b], cnt * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload ids");
+            ck(copy_to_device(d.d_m[b], d.h_m[b], cnt * sizeof(double)), "upload m");
+            ck(copy_to_device(d.d_id[b], d.h_id[b], cnt * sizeof(uint32_t)), "upload ids");
         }
     }
     initialized_ = true;

@@ -18,6 +18,7 @@
 // reads it (outputs, the C ABI), not every block; track snapshots are built
 // on the device (track.cu).
 #include "executor.h"
+#include "hostcopy.h"
 #include "interp.h"
 #include "parallel.h"
 #include "track.h"
@@ -345,7 +346,7 @@ void Executor::upload_particles(const std::vector<Vec3>& acc)
     std::vector<double> col(n);
     auto up = [&](double* dst, auto get) {
         for (size_t k = 0; k < n; k++) col[k] = get(k);
-        ck(cudaMemcpy(dst, col.data(), n * sizeof(double), cudaMemcpyHostToDevice), "upload particles");
+        ck(copy_to_device(dst, col.data(), n * sizeof(double)), "upload particles");
     };
     for (int b = 0; b < 2; b++) {
         glisser_particles& p = d_->buf[b].p;
@@ -358,9 +359,9 @@ void Executor::upload_particles(const std::vector<Vec3>& acc)
         up(p.ax, [&](size_t k) { return acc[k].x; });
         up(p.ay, [&](size_t k) { return acc[k].y; });
         up(p.az, [&](size_t k) { return acc[k].z; });
-        ck(cudaMemcpy(p.flags, pa_.flags.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice), "upload flags");
-        ck(cudaMemcpy(p.id, pa_.id.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload ids");
-        ck(cudaMemcpy(p.deathtime_index, pa_.deathtime_index.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice),
+        ck(copy_to_device(p.flags, pa_.flags.data(), n * sizeof(uint16_t)), "upload flags");
+        ck(copy_to_device(p.id, pa_.id.data(), n * sizeof(uint32_t)), "upload ids");
+        ck(copy_to_device(p.deathtime_index, pa_.deathtime_index.data(), n * sizeof(uint32_t)),
            "upload deathtime index");
     }
     host_dirty_ = false;
@@ -651,7 +652,7 @@ void Executor::init()
     }
     for (int b = 0; b < 2; b++) {
         ck(cudaMalloc(&d.d_log[b], log_bytes), "cudaMalloc log");
-        ck(cudaMemset(d.d_log[b], 0, log_bytes), "memset log");
+        ck(clear_on_device(d.d_log[b], log_bytes), "memset log");
         ck(cudaMalloc(&d.d_m[b], d.max_npl * sizeof(double)), "cudaMalloc m");
         ck(cudaMalloc(&d.d_rh[b], d.max_npl * sizeof(double)), "cudaMalloc rh");
         ck(cudaMalloc(&d.d_id[b], d.max_npl * sizeof(uint32_t)), "cudaMalloc id");

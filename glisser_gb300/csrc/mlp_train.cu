@@ -29,6 +29,7 @@
 #include <cstring>
 #include <stdexcept>
 
+#include "hostcopy.h"
 #include "kepler.cuh"
 #include "mlp_train.h"
 
@@ -513,7 +514,7 @@ void* mlp_upload(const std::vector<uint8_t>& file)
     MlpDev dev = make_dev(params.data(), h.norm);
     void* d = nullptr;
     if (cudaMalloc(&d, sizeof(MlpDev)) != cudaSuccess) throw std::bad_alloc();
-    if (cudaMemcpy(d, &dev, sizeof dev, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (copy_to_device(d, &dev, sizeof dev) != cudaSuccess) {
         cudaFree(d);
         throw std::runtime_error("learned-starter weights upload failed");
     }
@@ -553,10 +554,10 @@ MlpTrainer::MlpTrainer(size_t capacity, uint64_t seed) : cap_(capacity), params_
     check(cudaMalloc(&d_loss_, (MLP_NPARAM + 1) * sizeof(float)), "loss");
     check(cudaMalloc(&d_evals_, sizeof(unsigned long long)), "counter");
     check(cudaMalloc(&d_dev_, sizeof(MlpDev)), "weights");
-    check(cudaMemset(d_m_, 0, MLP_NPARAM * sizeof(float)), "memset");
-    check(cudaMemset(d_v_, 0, MLP_NPARAM * sizeof(float)), "memset");
-    check(cudaMemset(d_evals_, 0, sizeof(unsigned long long)), "memset");
-    check(cudaMemcpy(d_params_, params_.data(), MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice), "upload");
+    check(clear_on_device(d_m_, MLP_NPARAM * sizeof(float)), "memset");
+    check(clear_on_device(d_v_, MLP_NPARAM * sizeof(float)), "memset");
+    check(clear_on_device(d_evals_, sizeof(unsigned long long)), "memset");
+    check(copy_to_device(d_params_, params_.data(), MLP_NPARAM * sizeof(float)), "upload");
     check(cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(SM_FLOATS * sizeof(float))),
           "grad kernel attribute");
@@ -595,8 +596,8 @@ size_t MlpTrainer::log_states(const glisser_particles& pa, size_t n, double dt, 
             k++;
         }
         if (k > 0) {
-            check(cudaMemcpy(d_feat_ + 3 * n_, f.data(), 3 * k * sizeof(float), cudaMemcpyHostToDevice), "samples");
-            check(cudaMemcpy(d_target_ + n_, y.data(), k * sizeof(float), cudaMemcpyHostToDevice), "samples");
+            check(copy_to_device(d_feat_ + 3 * n_, f.data(), 3 * k * sizeof(float)), "samples");
+            check(copy_to_device(d_target_ + n_, y.data(), k * sizeof(float)), "samples");
         }
         m = k;
     }
@@ -607,8 +608,8 @@ size_t MlpTrainer::log_states(const glisser_particles& pa, size_t n, double dt, 
 void MlpTrainer::add_samples(const float* feat, const float* target, size_t n)
 {
     size_t m = std::min(n, cap_ - n_);
-    check(cudaMemcpy(d_feat_ + 3 * n_, feat, m * 3 * sizeof(float), cudaMemcpyHostToDevice), "samples");
-    check(cudaMemcpy(d_target_ + n_, target, m * sizeof(float), cudaMemcpyHostToDevice), "samples");
+    check(copy_to_device(d_feat_ + 3 * n_, feat, m * 3 * sizeof(float)), "samples");
+    check(copy_to_device(d_target_ + n_, target, m * sizeof(float)), "samples");
     n_ += m;
 }
 
@@ -672,9 +673,9 @@ void MlpTrainer::get_params(float* out) const { std::memcpy(out, params_.data(),
 void MlpTrainer::set_params(const float* in)
 {
     std::memcpy(params_.data(), in, MLP_NPARAM * sizeof(float));
-    check(cudaMemcpy(d_params_, params_.data(), MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice), "upload");
-    check(cudaMemset(d_m_, 0, MLP_NPARAM * sizeof(float)), "memset");
-    check(cudaMemset(d_v_, 0, MLP_NPARAM * sizeof(float)), "memset");
+    check(copy_to_device(d_params_, params_.data(), MLP_NPARAM * sizeof(float)), "upload");
+    check(clear_on_device(d_m_, MLP_NPARAM * sizeof(float)), "memset");
+    check(clear_on_device(d_v_, MLP_NPARAM * sizeof(float)), "memset");
     adam_t_ = 0;
     dev_stale_ = true;
 }
@@ -749,8 +750,8 @@ void MlpTrainer::gradients(const float* feat, const float* target, size_t n, flo
     check(cudaMalloc(&dtg, n * sizeof(float)), "samples");
     const uint32_t blocks = (uint32_t)((n + TT - 1) / TT);
     try {
-        check(cudaMemcpy(df, feat, n * 3 * sizeof(float), cudaMemcpyHostToDevice), "samples");
-        check(cudaMemcpy(dtg, target, n * sizeof(float), cudaMemcpyHostToDevice), "samples");
+        check(copy_to_device(df, feat, n * 3 * sizeof(float)), "samples");
+        check(copy_to_device(dtg, target, n * sizeof(float)), "samples");
         ensure_partials(blocks);
         grad_launch(df, dtg, (uint32_t)n, (uint32_t)n, true, 0, 0, blocks);
         AdamArgs a;
@@ -778,7 +779,7 @@ const MlpDev* MlpTrainer::device_weights()
 {
     if (dev_stale_) {
         MlpDev d = make_dev(params_.data(), norm);
-        check(cudaMemcpy(d_dev_, &d, sizeof d, cudaMemcpyHostToDevice), "weights");
+        check(copy_to_device(d_dev_, &d, sizeof d), "weights");
         dev_stale_ = false;
     }
     return reinterpret_cast<const MlpDev*>(d_dev_);
@@ -791,7 +792,7 @@ void MlpTrainer::predict(const float* feat, size_t n, float* y)
     float *df = nullptr, *dy = nullptr;
     check(cudaMalloc(&df, n * 3 * sizeof(float)), "features");
     check(cudaMalloc(&dy, n * sizeof(float)), "outputs");
-    cudaError_t e = cudaMemcpy(df, feat, n * 3 * sizeof(float), cudaMemcpyHostToDevice);
+    cudaError_t e = copy_to_device(df, feat, n * 3 * sizeof(float));
     if (e == cudaSuccess) {
         predict_kernel<<<(unsigned)((n + 127) / 128), 128, 0, stream_>>>(w, df, (uint32_t)n, dy);
         e = cudaGetLastError();
