@@ -566,7 +566,7 @@ MlpTrainer::MlpTrainer(size_t capacity, uint64_t seed) : cap_(capacity), params_
 MlpTrainer::~MlpTrainer()
 {
     cudaFree(d_feat_); cudaFree(d_target_); cudaFree(d_params_); cudaFree(d_m_); cudaFree(d_v_);
-    cudaFree(d_partials_); cudaFree(d_loss_); cudaFree(d_evals_); cudaFree(d_dev_);
+    cudaFree(d_partials_); cudaFree(d_loss_); cudaFree(d_losses_); cudaFree(d_evals_); cudaFree(d_dev_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -685,8 +685,20 @@ void MlpTrainer::ensure_partials(size_t blocks)
     if (blocks <= partials_cap_) return;
     cudaFree(d_partials_);
     d_partials_ = nullptr;
+    partials_cap_ = 0;
     check(cudaMalloc(&d_partials_, blocks * PART * sizeof(float)), "partials");
     partials_cap_ = blocks;
+}
+
+// Kept from run to run: cudaFree waits for the whole device.
+void MlpTrainer::ensure_losses(size_t steps)
+{
+    if (steps <= losses_cap_) return;
+    cudaFree(d_losses_);
+    d_losses_ = nullptr;
+    losses_cap_ = 0;
+    check(cudaMalloc(&d_losses_, steps * sizeof(float)), "losses");
+    losses_cap_ = steps;
 }
 
 void MlpTrainer::grad_launch(const float* feat, const float* target, uint32_t n, uint32_t batch, bool sequential,
@@ -712,12 +724,7 @@ void MlpTrainer::train(int steps, int batch, float lr, float lr_min, uint64_t se
     if (steps < 0 || batch < TT || batch % TT != 0) throw std::invalid_argument("train: batch must be a multiple of 128");
     const uint32_t blocks = (uint32_t)(batch / TT);
     ensure_partials(blocks);
-    // the losses of the run, one per step
-    struct DeviceFloats {
-        float* p = nullptr;
-        ~DeviceFloats() { cudaFree(p); }
-    } dl;
-    if (losses && steps > 0) check(cudaMalloc(&dl.p, (size_t)steps * sizeof(float)), "losses");
+    if (losses) ensure_losses((size_t)steps);
     const float b1 = 0.9f, b2 = 0.999f;
     for (int s = 0; s < steps; s++) {
         grad_launch(d_feat_, d_target_, (uint32_t)n_, (uint32_t)batch, false, seed, (uint32_t)s, blocks);
@@ -733,11 +740,13 @@ void MlpTrainer::train(int steps, int batch, float lr, float lr_min, uint64_t se
         a.inv_batch = 1.0f / (float)batch;
         a.apply = 1;
         check(launch_early(adam_kernel, MLP_NPARAM / ADAM_THREADS + 1, ADAM_THREADS, 0, stream_, d_params_, d_m_, d_v_,
-                           (const float*)d_partials_, blocks, a, (float*)nullptr, dl.p ? dl.p + s : (float*)nullptr),
+                           (const float*)d_partials_, blocks, a, (float*)nullptr,
+                           losses ? d_losses_ + s : (float*)nullptr),
               "adam_kernel");
     }
     check(cudaStreamSynchronize(stream_), "training");
-    if (dl.p) check(cudaMemcpy(losses, dl.p, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost), "losses");
+    if (losses && steps > 0)
+        check(cudaMemcpy(losses, d_losses_, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost), "losses");
     check(cudaMemcpy(params_.data(), d_params_, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost), "parameters");
     dev_stale_ = true;
 }

@@ -81,9 +81,10 @@ private:
     size_t cap_, n_ = 0;
     float *d_feat_ = nullptr, *d_target_ = nullptr;
     float *d_params_ = nullptr, *d_m_ = nullptr, *d_v_ = nullptr, *d_partials_ = nullptr, *d_loss_ = nullptr;
+    float* d_losses_ = nullptr;                 // the losses of a training run, one per step
     unsigned long long* d_evals_ = nullptr;
     void* d_dev_ = nullptr;
-    size_t partials_cap_ = 0;
+    size_t partials_cap_ = 0, losses_cap_ = 0;
     std::vector<float> params_;
     bool dev_stale_ = true;
     int adam_t_ = 0;
@@ -91,6 +92,7 @@ private:
     cudaStream_t stream_ = nullptr;
 
     void ensure_partials(size_t blocks);
+    void ensure_losses(size_t steps);
     void grad_launch(const float* feat, const float* target, uint32_t n, uint32_t batch, bool sequential,
                      uint64_t seed, uint32_t step, uint32_t blocks);
 };

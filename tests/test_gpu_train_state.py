@@ -1,5 +1,6 @@
 """Training runs that follow one another on one trainer: parameters set by the caller
-start a run with cleared Adam moments, whatever ran before."""
+start a run with cleared Adam moments, whatever ran before, and each run returns its
+own losses."""
 import numpy as np
 import pytest
 
@@ -37,3 +38,15 @@ def test_set_parameters_start_a_fresh_run():
         a.params = p
         losses = a.train(20, batch=256, lr=1e-2, seed=5)
         assert np.array_equal(losses, want_losses) and np.array_equal(a.params, want)
+
+
+def test_losses_of_runs_of_different_lengths():
+    # the trainer's loss buffer grows with the longest run and is used again
+    a = trainer()
+    p = a.params.copy()
+    for steps in (1, 50, 3, 50, 49):
+        a.params = p
+        got = a.train(steps, batch=256, lr=1e-2, seed=steps)
+        b = trainer()
+        b.params = p
+        assert np.array_equal(got, b.train(steps, batch=256, lr=1e-2, seed=steps))
