@@ -105,12 +105,16 @@ __device__ __forceinline__ ff ff_sqr3(ff x, ff y, ff z) { return ff_sum3(ff_sqr_
 // The rare halves of ff_split_fast and ff_widen, as calls: inlined, the compiler
 // turns their branches into predicated instructions that every step issues
 // (ff_widen's FP64 conversions and addition, so issued, made the crossers'
-// block 1.9x longer).
+// block 1.9x longer).  Zero is not left to them: a planar swarm's z is zero at
+// every step.  No FP64 instruction in the split's.
 static __device__ __noinline__ ff ff_split_rare(double d)
 {
-    if (d != d) return { __int_as_float(0x7fc00000), __int_as_float(0x7fc00000) };
-    if (fabs(d) >= 0x1p128) return { f32_trunc(d), 0.0f };      // infinity
-    return ff_split(d);
+    const unsigned e = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+    ff f = ff_split(d);                       // infinite from 2^128 on, for NaN too
+    if (e >= 1023u + 128u) f.lo = 0.0f;
+    const unsigned m = ((unsigned)__double2hiint(d) << 12) | (unsigned)__double2loint(d);
+    if (e == 0x7ffu && m != 0u) f.hi = f.lo = __int_as_float(0x7fc00000);
+    return f;
 }
 static __device__ __noinline__ double ff_widen_rare(float hi, float lo) { return (double)hi + (double)lo; }
 
@@ -146,6 +150,13 @@ __device__ __forceinline__ ff ff_split_fast(double d)
     return split_common(d);
 }
 
+// A rare one of three components.
+__device__ __forceinline__ ff split_uncommon(double d)
+{
+    if ((((unsigned)__double2hiint(d) & 0x7fffffffu) | (unsigned)__double2loint(d)) == 0u) return { 0.0f, 0.0f };
+    return ff_split_rare(d);
+}
+
 // Three at once, with one branch for the rare ones.
 __device__ __forceinline__ void ff_split3(double x, double y, double z, ff& fx, ff& fy, ff& fz)
 {
@@ -153,9 +164,9 @@ __device__ __forceinline__ void ff_split3(double x, double y, double z, ff& fx, 
     fy = split_common(y);
     fz = split_common(z);
     if (split_is_rare(x) || split_is_rare(y) || split_is_rare(z)) {
-        fx = ff_split_rare(x);
-        fy = ff_split_rare(y);
-        fz = ff_split_rare(z);
+        if (split_is_rare(x)) fx = split_uncommon(x);
+        if (split_is_rare(y)) fy = split_uncommon(y);
+        if (split_is_rare(z)) fz = split_uncommon(z);
     }
 }
 
@@ -187,15 +198,21 @@ __device__ __forceinline__ double ff_widen(ff x)
     return widen_common(x);
 }
 
+__device__ __forceinline__ double widen_uncommon(ff x)
+{
+    if (x.hi == 0.0f && x.lo == 0.0f) return 0.0;
+    return ff_widen_rare(x.hi, x.lo);
+}
+
 __device__ __forceinline__ void ff_widen3(ff x, ff y, ff z, double& dx, double& dy, double& dz)
 {
     dx = widen_common(x);
     dy = widen_common(y);
     dz = widen_common(z);
     if (widen_is_rare(x) || widen_is_rare(y) || widen_is_rare(z)) {
-        dx = ff_widen_rare(x.hi, x.lo);
-        dy = ff_widen_rare(y.hi, y.lo);
-        dz = ff_widen_rare(z.hi, z.lo);
+        if (widen_is_rare(x)) dx = widen_uncommon(x);
+        if (widen_is_rare(y)) dy = widen_uncommon(y);
+        if (widen_is_rare(z)) dz = widen_uncommon(z);
     }
 }
 
