@@ -21,7 +21,7 @@ struct Common {
     double outer2;
     double tol_dt;          // Kepler residual tolerance x dt
     SmallStepDt sdt;        // the step's constants of the small-step drift
-    float dt_range;         // dt within the range those constants cover: 1, else NaN (the general drift runs)
+    bool dt_range;          // dt within the range those constants cover
     float r2_hi;            // |r|^2 above which the radius tests and ranges are looked at one by one
     int starter;
     int kill;
@@ -124,6 +124,7 @@ struct CtaShared {
     PlanetConst pk[MAX_PLANETS];
     ff muh, mudt;               // mu dt^2 / 2, mu dt
     float r2_lo;                // |r|^2 below which the Sun's radius test is looked at
+    bool tiers;                 // the float-float drift's tiers cover this system's units and step
     uint64_t bar[2];
     int abort;
     uint32_t item;
@@ -220,10 +221,11 @@ __device__ __forceinline__ void planet_kick64(const double* L, int j, double rx,
 // buffers.  `phase` counts completed waits per buffer (identical in every
 // thread; carried across tiles of a persistent CTA).  Returns false after a
 // staging timeout.  KICK64: the planet kick and its radius tests in FP64
-// (planet_kick64) instead of float-float.
-template <int NP, int CTA, int PPT, bool LEARNED, bool KICK64, int NET_ROWS = MLP_ROWS, int NET_QU = 1>
-__device__ __forceinline__ bool run_tile(const Common& p, const double* log, uint32_t first, uint32_t count,
-                                         double* stage, CtaShared& sh, uint32_t* phase)
+// (planet_kick64) instead of float-float.  TIERS: each drift in the float-float
+// tier that takes it, else general; without, every drift general.
+template <bool TIERS, int NP, int CTA, int PPT, bool LEARNED, bool KICK64, int NET_ROWS = MLP_ROWS, int NET_QU = 1>
+__device__ __forceinline__ bool run_tile_as(const Common& p, const double* log, uint32_t first, uint32_t count,
+                                            double* stage, CtaShared& sh, uint32_t* phase)
 {
     const int np = NP > 0 ? NP : (int)p.npl - 1;
     const uint32_t rec = 3u * (uint32_t)(np + 1);
@@ -276,12 +278,18 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
             vy[k] = fma(a0y, hdt, vy[k]);
             vz[k] = fma(a0z, hdt, vz[k]);
         }
-        ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
-        f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
-        fri[k] = ff_rsqrt(f2[k]);
-        if (!(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX)) fri[k].hi = __int_as_float(0x7fc00000);
-        r2[k] = rinv[k] = 0;
-        general[k] = false;
+        r2[k] = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
+        if constexpr (TIERS) {
+            ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
+            f2[k] = ff_split_fast(r2[k]);
+            fri[k] = ff_rsqrt(f2[k]);
+            if (!(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX)) fri[k].hi = __int_as_float(0x7fc00000);
+            r2[k] = rinv[k] = 0;
+            general[k] = false;
+        } else {
+            rinv[k] = rsqrt_lean(r2[k]);
+            general[k] = true;
+        }
     }
 
     bool ok = true;
@@ -328,69 +336,80 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                 ff wx, wy, wz;
                 // this step's velocity change beyond vx..vz, summed with the kick's
                 ff gx = { 0.0f, 0.0f }, gy = { 0.0f, 0.0f }, gz = { 0.0f, 0.0f };
-                // tau^2 / 2 in FP32 first: a wide drift costs the small-step one five instructions
-                const float q3 = sh.muh.hi * fri[k].hi * (fri[k].hi * fri[k].hi);
-                int tier = DRIFT_GENERAL;
-                if (p.starter != STARTER_CLASSIC && q3 < 0.5f * SMALL_DRIFT_TAU2) {
-                    ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
-                    tier = small_drift<false>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
-                }
-                if (tier == DRIFT_SMALL) {
-                    // r' = r + dt v + ((f - 1) r + (g - dt) v): dt v in FP64, the rest a
-                    // float-float correction
-                    const ff cx = ff_norm(ff_add_u(ff_mul_u(sd.f1, fx[k]), ff_mul_u(sd.gdt, wx)));
-                    const ff cy = ff_norm(ff_add_u(ff_mul_u(sd.f1, fy[k]), ff_mul_u(sd.gdt, wy)));
-                    const ff cz = ff_norm(ff_add_u(ff_mul_u(sd.f1, fz[k]), ff_mul_u(sd.gdt, wz)));
-                    double dx, dy, dz;
-                    ff_widen3(cx, cy, cz, dx, dy, dz);
-                    rx[k] += fma(p.dt, vx[k], dx);
-                    ry[k] += fma(p.dt, vy[k], dy);
-                    rz[k] += fma(p.dt, vz[k], dz);
-                    const ff ox = fx[k], oy = fy[k], oz = fz[k];
-                    ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
-                    // |r'|^2 in FP64 (three instructions of a pipe with room), then
-                    // 1/|r'| in float-float
-                    f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
-                    fri[k] = ff_rsqrt(f2[k]);
-                    // v' = v + (fd r + (gd - 1) v)
-                    const ff gd1 = ff_neg(ff_mul_u(sd.h, fri[k]));
-                    const ff fd = ff_mul_u(sd.fdr, fri[k]);
-                    gx = ff_add_u(ff_mul_u(fd, ox), ff_mul_u(gd1, wx));
-                    gy = ff_add_u(ff_mul_u(fd, oy), ff_mul_u(gd1, wy));
-                    gz = ff_add_u(ff_mul_u(fd, oz), ff_mul_u(gd1, wz));
-                    general[k] = false;
-                    evals++;
-                } else {
-                    if (!general[k]) {
-                        r2[k] = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
-                        rinv[k] = rsqrt_lean(r2[k]);
-                        general[k] = true;
-                    }
+                // the general drift, from r2, rinv
+                auto solve = [&](GFun& g) {
+                    const DriftInvariants q =
+                        drift_invariants(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], p.dt, mu);
+                    const DriftResult d = kepler_solve<LEARNED, NET_ROWS, NET_QU>(g, rinv[k], q, p.dt, mu, p.starter,
+                                                                                  p.mlp, p.tol_dt);
+                    fl = d.flags;
+                    evals += d.evals;
+                    if constexpr (LEARNED) nets += d.net;
+                    wide += d.wide;
+                    return q.mu_r;
+                };
+                if constexpr (!TIERS) {
                     GFun g;
-                    double mu_r;
-                    if (p.starter != STARTER_CLASSIC && q3 < 0.5f * MEDIUM_DRIFT_TAU2) {
+                    const double mu_r = solve(g);
+                    drift_apply(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], g, mu_r, p.dt, mu);
+                    if constexpr (!KICK64) ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
+                } else {
+                    // tau^2 / 2 in FP32 first: a wide drift costs the small-step one five instructions
+                    const float q3 = sh.muh.hi * fri[k].hi * (fri[k].hi * fri[k].hi);
+                    int tier = DRIFT_GENERAL;
+                    if (q3 < 0.5f * SMALL_DRIFT_TAU2) {
                         ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
-                        tier = small_drift<true>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
+                        tier = small_drift<false>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
                     }
-                    if (tier == DRIFT_MEDIUM) {
-                        mu_r = mu * rinv[k];
-                        medium_gfuns(sd, p.dt * rinv[k], g.g1, g.g2, g.g3);
+                    if (tier == DRIFT_SMALL) {
+                        // r' = r + dt v + ((f - 1) r + (g - dt) v): dt v in FP64, the rest a
+                        // float-float correction
+                        const ff cx = ff_norm(ff_add_u(ff_mul_u(sd.f1, fx[k]), ff_mul_u(sd.gdt, wx)));
+                        const ff cy = ff_norm(ff_add_u(ff_mul_u(sd.f1, fy[k]), ff_mul_u(sd.gdt, wy)));
+                        const ff cz = ff_norm(ff_add_u(ff_mul_u(sd.f1, fz[k]), ff_mul_u(sd.gdt, wz)));
+                        double dx, dy, dz;
+                        ff_widen3(cx, cy, cz, dx, dy, dz);
+                        rx[k] += fma(p.dt, vx[k], dx);
+                        ry[k] += fma(p.dt, vy[k], dy);
+                        rz[k] += fma(p.dt, vz[k], dz);
+                        const ff ox = fx[k], oy = fy[k], oz = fz[k];
+                        ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
+                        // |r'|^2 in FP64 (three instructions of a pipe with room), then
+                        // 1/|r'| in float-float
+                        f2[k] = ff_split_fast(fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])));
+                        fri[k] = ff_rsqrt(f2[k]);
+                        // v' = v + (fd r + (gd - 1) v)
+                        const ff gd1 = ff_neg(ff_mul_u(sd.h, fri[k]));
+                        const ff fd = ff_mul_u(sd.fdr, fri[k]);
+                        gx = ff_add_u(ff_mul_u(fd, ox), ff_mul_u(gd1, wx));
+                        gy = ff_add_u(ff_mul_u(fd, oy), ff_mul_u(gd1, wy));
+                        gz = ff_add_u(ff_mul_u(fd, oz), ff_mul_u(gd1, wz));
+                        general[k] = false;
                         evals++;
                     } else {
-                        const DriftInvariants q =
-                            drift_invariants(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], p.dt, mu);
-                        const DriftResult d = kepler_solve<LEARNED, NET_ROWS, NET_QU>(g, rinv[k], q, p.dt, mu, p.starter,
-                                                                                      p.mlp, p.tol_dt);
-                        mu_r = q.mu_r;
-                        fl = d.flags;
-                        evals += d.evals;
-                        if constexpr (LEARNED) nets += d.net;
-                        wide += d.wide;
+                        if (!general[k]) {
+                            r2[k] = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
+                            rinv[k] = rsqrt_lean(r2[k]);
+                            general[k] = true;
+                        }
+                        GFun g;
+                        double mu_r;
+                        if (q3 < 0.5f * MEDIUM_DRIFT_TAU2) {
+                            ff_split3(vx[k], vy[k], vz[k], wx, wy, wz);
+                            tier = small_drift<true>(fx[k], fy[k], fz[k], wx, wy, wz, f2[k], fri[k], sh.muh, sh.mudt, p.sdt, sd);
+                        }
+                        if (tier == DRIFT_MEDIUM) {
+                            mu_r = mu * rinv[k];
+                            medium_gfuns(sd, p.dt * rinv[k], g.g1, g.g2, g.g3);
+                            evals++;
+                        } else {
+                            mu_r = solve(g);
+                        }
+                        drift_apply(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], g, mu_r, p.dt, mu);
+                        ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
+                        f2[k] = ff_split_fast(r2[k]);
+                        fri[k] = ff_split_fast(rinv[k]);
                     }
-                    drift_apply(rx[k], ry[k], rz[k], vx[k], vy[k], vz[k], r2[k], rinv[k], g, mu_r, p.dt, mu);
-                    ff_split3(rx[k], ry[k], rz[k], fx[k], fy[k], fz[k]);
-                    f2[k] = ff_split_fast(r2[k]);
-                    fri[k] = ff_split_fast(rinv[k]);
                 }
                 double aax, aay, aaz;
                 ff sx, sy, sz;
@@ -410,19 +429,23 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                     if constexpr (NP > 0) {
                         // unrolled up to four planets: 2 % faster than rolled on the
                         // giants (47.5 against 48.5 ms) since the kernel is bound by issue
-#pragma unroll (NP <= 4 ? NP : 1)
+#pragma unroll (TIERS && NP <= 4 ? NP : 1)
                         for (int j = 1; j <= NP; j++) planet_kick(L, j, fx[k], fy[k], fz[k], sx, sy, sz, fl, border, sh);
                     } else {
                         for (int j = 1; j <= np; j++) planet_kick(L, j, fx[k], fy[k], fz[k], sx, sy, sz, fl, border, sh);
                     }
                 }
-                if (!(f2[k].hi > sh.r2_lo && f2[k].hi < p.r2_hi)) {
+                bool near_radius = true;
+                if constexpr (TIERS) near_radius = !(f2[k].hi > sh.r2_lo && f2[k].hi < p.r2_hi);
+                if (near_radius) {
                     // near or beyond a radius, or outside the float-float range
-                    const double rr = fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k]));
+                    const double rr =
+                        TIERS ? fma(rx[k], rx[k], fma(ry[k], ry[k], rz[k] * rz[k])) : r2[k];
                     border += near_nonneg(rr, rh2_sun) + near_nonneg(rr, p.outer2);
                     if (lt_nonneg(rr, rh2_sun)) fl = 0x0001;
                     if (gt_nonneg(rr, p.outer2)) fl = 0x0002;
-                    if (!(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX)) fri[k].hi = __int_as_float(0x7fc00000);
+                    if (TIERS && !(f2[k].hi > KICK_R2_MIN && f2[k].hi < KICK_R2_MAX))
+                        fri[k].hi = __int_as_float(0x7fc00000);
                 }
                 flags[k] = fl;
                 const uint32_t step = cfirst + s + 1;
@@ -442,11 +465,17 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
                 }
                 if constexpr (KICK64) {
                     const double kc = last ? hdt : p.dt;
-                    double dx, dy, dz;
-                    ff_widen3(ff_norm(gx), ff_norm(gy), ff_norm(gz), dx, dy, dz);
-                    vx[k] += fma(aax, kc, dx);
-                    vy[k] += fma(aay, kc, dy);
-                    vz[k] += fma(aaz, kc, dz);
+                    if constexpr (TIERS) {
+                        double dx, dy, dz;
+                        ff_widen3(ff_norm(gx), ff_norm(gy), ff_norm(gz), dx, dy, dz);
+                        vx[k] += fma(aax, kc, dx);
+                        vy[k] += fma(aay, kc, dy);
+                        vz[k] += fma(aaz, kc, dz);
+                    } else {
+                        vx[k] = fma(aax, kc, vx[k]);
+                        vy[k] = fma(aay, kc, vy[k]);
+                        vz[k] = fma(aaz, kc, vz[k]);
+                    }
                 } else {
                     double dx, dy, dz;
                     ff_widen3(ff_norm(ff_add_u(gx, sx)), ff_norm(ff_add_u(gy, sy)), ff_norm(ff_add_u(gz, sz)), dx, dy,
@@ -544,6 +573,26 @@ __device__ __forceinline__ bool run_tile(const Common& p, const double* log, uin
     return ok;
 }
 
+// The tiers' loop, or the general drift's alone where every step is general (sh.tiers,
+// uniform over the CTA): a straight line.  With the tiers' tests, splits and
+// branches around the general drift, 4,000 particles near planets' orbits with the
+// classic starter and the FP64 kick took 795 us for 128 steps, here 659; 150,000 with
+// giants in kilometres and seconds 3,099 and 2,746 us, with the FP64 kick 4,509 and
+// 3,899.  The learned kernels keep the one loop (a NaN in muh makes their drifts
+// general): a second copy of the network made their 100,000 close-eccentric
+// particles x 256 steps 6.7 -> 7.5 ms, as a call 8.4.
+template <int NP, int CTA, int PPT, bool LEARNED, bool KICK64, int NET_ROWS = MLP_ROWS, int NET_QU = 1>
+__device__ __forceinline__ bool run_tile(const Common& p, const double* log, uint32_t first, uint32_t count,
+                                         double* stage, CtaShared& sh, uint32_t* phase)
+{
+    if constexpr (!LEARNED) {
+        if (!sh.tiers)
+            return run_tile_as<false, NP, CTA, PPT, LEARNED, KICK64, NET_ROWS, NET_QU>(p, log, first, count, stage, sh,
+                                                                                      phase);
+    }
+    return run_tile_as<true, NP, CTA, PPT, LEARNED, KICK64, NET_ROWS, NET_QU>(p, log, first, count, stage, sh, phase);
+}
+
 __device__ __forceinline__ void load_planet_constants(const Common& p, CtaShared& sh, uint32_t npl, const double* m,
                                                       const double* rh, const uint32_t* pid)
 {
@@ -566,9 +615,10 @@ __device__ __forceinline__ void load_planet_constants(const Common& p, CtaShared
             const SmallStepMu c = small_step_mu(m[0], p.dt);
             sh.muh = c.muh;
             sh.mudt = c.mudt;
-            // outside the range the constant's products cover, NaN: the general drift runs
-            if (!(sh.muh.hi > 0x1p-40f && sh.muh.hi < 0x1p30f)) sh.muh.hi = __int_as_float(0x7fc00000);
-            sh.muh.hi *= p.dt_range;
+            // outside the range the constants' products cover, and with the classic
+            // starter, the general drift runs at every step
+            sh.tiers = p.dt_range && sh.muh.hi > 0x1p-40f && sh.muh.hi < 0x1p30f && p.starter != STARTER_CLASSIC;
+            if (!sh.tiers) sh.muh.hi = __int_as_float(0x7fc00000);
             sh.r2_lo = near;
         }
     }
@@ -606,7 +656,7 @@ inline bool fill_common(Common& p, const glisser_particles* pa, const glisser_st
     p.sdt.dt2 = ff_of(sp->dt * sp->dt);
     p.sdt.dt_half = ff_of(0.5 * sp->dt);
     p.sdt.neg_dt = ff_of(-sp->dt);
-    p.dt_range = sp->dt > 0x1p-24 && sp->dt < 0x1p24 ? 1.0f : std::nanf("");
+    p.dt_range = sp->dt > 0x1p-24 && sp->dt < 0x1p24;
     p.tol_dt = (sp->kepler_tol > 0 ? sp->kepler_tol : KEP_TOL) * sp->dt;
     p.starter = sp->starter;
     p.kill = sp->kill_encounters;
