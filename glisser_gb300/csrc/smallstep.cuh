@@ -48,12 +48,16 @@ namespace glisser {
 constexpr float SMALL_DRIFT_TAU2 = 1e-3f;
 constexpr float MEDIUM_DRIFT_TAU2 = 1e-2f;
 
-// Least tau^2 / 2 of a small step: 4,400 au at dt = 180 d.  It only keeps the chain
-// of products within a float's range; a bound of 2^-30 (1,700 au) left one particle
-// in 500 of a scattered disk to the general drift at every step, and each held its
-// warp: 1,000 particles x 128 steps 706 us there, 449 here (620 with every drift
-// general), 16,000 867 and 604, 500,000 5.12 and 4.23 ms.
-constexpr float TINY_DRIFT_TH = 0x1p-34f;
+// Least tau^2 / 2 of a small step.  It only keeps the chain of products within a
+// float's range: 2^-34 does for any mu, dt and r, and where the ranges of these
+// are checked (run_tile: |r|^2 in 2^-40..2^44, mu dt^2 / 2 in 2^-40..2^30, dt in
+// 2^-24..2^24) tau^2 / 2 is 2^-106 at least, and what underflows is below 2^-70 of what
+// it is added to.  A particle below the bound takes the general drift at every step and
+// holds its warp: with 2^-30 (1,700 au at dt = 180 d), one in 500 of a scattered disk,
+// 1,000 particles x 128 steps took 706 us, with 2^-34 449, 16,000 867 and 604, 500,000
+// 5.12 and 4.23 ms; and with 2^-34 150,000 at dt = 10 d, where it lies at 630 au, took
+// 2.53 ms (1.74 with every drift general, 0.66 without a bound).
+constexpr float TINY_DRIFT_TH = 0x1p-34f, FAR_DRIFT_TH = 0x1p-110f;
 
 // --- float-float without the renormalising step: hi + lo with |lo| up to a
 // few units in hi's last place.  Sums and products of them lose ~2^-46; a
@@ -264,6 +268,7 @@ __device__ __forceinline__ ff ff_rcp(ff x)
 // Constants of a launch's step dt.
 struct SmallStepDt {
     ff dt2, dt_half, neg_dt;      // dt^2, dt / 2, -dt
+    float th_min = TINY_DRIFT_TH; // the least tau^2 / 2: FAR_DRIFT_TH where the ranges are checked
 };
 
 // Constants of the central mass mu and the step dt: mu dt^2 / 2, mu dt.  Rounded
@@ -325,7 +330,7 @@ __device__ __forceinline__ float kepler_residual(ff X, ff Y, float w, ff q2, ff 
 // the ensembles 5 %.  The line at 1e-2: e, q2 and q3 at 2^-46 then change
 // r by 2^-55 and v by 2^-53 at most, and the series end below 2^-46.  300,000
 // scattered-disk particles x 256 steps, 0.9 % of their drifts here and 0.1 % beyond,
-// but spread over the warps: 7.19 -> 6.47 ms (5.15 with TINY_DRIFT_TH), error against long double 3.1e-15 before
+// but spread over the warps: 7.19 -> 6.47 ms (5.15 with tau^2 / 2 down to 2^-34), error against long double 3.1e-15 before
 // and after; 1e6 particles x 64 steps with the learned starter
 // 5.94 -> 5.21 ms.
 template <bool MEDIUM>
@@ -346,7 +351,7 @@ __device__ __forceinline__ int small_drift(ff rx, ff ry, ff rz, ff vx, ff vy, ff
     const ff A = ff_add_u(ff_scale(th, 4.0f), ff_neg(b));
     const ff Y = ff_mul_u(ff_add_u(b, ff_scale(th, -2.0f)), ff_sixth());
     const float a = A.hi, x = X.hi, y = Y.hi;
-    const bool inside = th.hi < 0.5f * (MEDIUM ? MEDIUM_DRIFT_TAU2 : SMALL_DRIFT_TAU2) && th.hi > TINY_DRIFT_TH &&
+    const bool inside = th.hi < 0.5f * (MEDIUM ? MEDIUM_DRIFT_TAU2 : SMALL_DRIFT_TAU2) && th.hi > c.th_min &&
                         a > 0x1p-20f * th.hi;
     if (!inside) return DRIFT_GENERAL;
 

@@ -656,6 +656,7 @@ inline bool fill_common(Common& p, const glisser_particles* pa, const glisser_st
     p.sdt.dt2 = ff_of(sp->dt * sp->dt);
     p.sdt.dt_half = ff_of(0.5 * sp->dt);
     p.sdt.neg_dt = ff_of(-sp->dt);
+    p.sdt.th_min = FAR_DRIFT_TH;       // the ranges: dt_range here, mu dt^2 in load_planet_constants, |r|^2 in run_tile
     p.dt_range = sp->dt > 0x1p-24 && sp->dt < 0x1p24;
     p.tol_dt = (sp->kepler_tol > 0 ? sp->kepler_tol : KEP_TOL) * sp->dt;
     p.starter = sp->starter;
