@@ -466,8 +466,9 @@ __device__ __forceinline__ bool run_tile_as(const Common& p, const double* log, 
                 if constexpr (KICK64) {
                     const double kc = last ? hdt : p.dt;
                     if constexpr (TIERS) {
-                        double dx, dy, dz;
-                        ff_widen3(ff_norm(gx), ff_norm(gy), ff_norm(gz), dx, dy, dz);
+                        // (a general step's gx..gz are zero, which would take the rare branch)
+                        double dx = 0, dy = 0, dz = 0;
+                        if (!general[k]) ff_widen3(ff_norm(gx), ff_norm(gy), ff_norm(gz), dx, dy, dz);
                         vx[k] += fma(aax, kc, dx);
                         vy[k] += fma(aay, kc, dy);
                         vz[k] += fma(aaz, kc, dz);
