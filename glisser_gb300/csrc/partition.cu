@@ -14,7 +14,7 @@
 // tile's before this one's is written, so that loads are in flight across the
 // barriers.  A separate scan launch of one CTA between the two (per-tile
 // counts, one particle per thread, the record read after the ranks) took 55 us
-// for 1e6 particles and 197 us for 4e6; this takes 35 and 119 us, 0.76 and 0.89
+// for 1e6 particles and 197 us for 4e6; this takes 36.9 and 119 us, 0.72 and 0.89
 // of the measured copy rate, and 8.4 against 14.5 us for 5,000.
 #include <cuda.h>
 

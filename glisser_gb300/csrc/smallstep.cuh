@@ -33,8 +33,8 @@
 // |v| against 7e-17 for the coefficients correctly rounded); at 1e-3..2e-3 it is
 // 3.4e-16.  Measured on GB300, before (every drift general) and after: 1e6
 // particles x 1,024 steps with four giants 98.6 -> 45.5 ms; 2e6 planet crossers
-// x 100 steps 16.6 -> 5.8 ms; 2,000 particles x 128 steps 643 -> 336 us;
-// 256 ensembles, 1.5e6 particles x 512 steps, 80 -> 37.3 ms.  Position error of
+// x 100 steps 16.6 -> 5.8 ms; 2,000 particles x 128 steps 643 -> 333 us;
+// 256 ensembles, 1.5e6 particles x 512 steps, 80 -> 35.5 ms.  Position error of
 // those blocks against long double: giants 1.49e-14 -> 1.01e-14 rms, belt
 // 2.34e-14 -> 1.64e-14, crossers 8.6e-16 -> 7.2e-16, scattered disk
 // 3.5e-15 -> 3.0e-15.
@@ -44,7 +44,12 @@
 namespace glisser {
 
 // Bounds on tau^2 of the small-step drift and of its solution of Kepler's
-// equation for a drift applied in FP64.
+// equation for a drift applied in FP64.  A warp that holds drifts on both sides of
+// a bound runs both paths.  Where most warps do, around 1e-3, that gives back the
+// gain: 150,000 belt particles x 128 steps take 0.67 ms at dt = 300 d (1.74 with every
+// drift general), 1.86 at 600 d, tau^2 of 6e-4 to 2e-3 (1.80), 1.34 at 900 d (2.30);
+// with the FP64 kick 1.10 (2.15), 2.38 (2.22), 1.89 (2.73); 4,000 with the FP64
+// kick at 600 d 686 us (568).
 constexpr float SMALL_DRIFT_TAU2 = 1e-3f;
 constexpr float MEDIUM_DRIFT_TAU2 = 1e-2f;
 
@@ -56,7 +61,7 @@ constexpr float MEDIUM_DRIFT_TAU2 = 1e-2f;
 // holds its warp: with 2^-30 (1,700 au at dt = 180 d), one in 500 of a scattered disk,
 // 1,000 particles x 128 steps took 706 us, with 2^-34 449, 16,000 867 and 604, 500,000
 // 5.12 and 4.23 ms; and with 2^-34 150,000 at dt = 10 d, where it lies at 630 au, took
-// 2.53 ms (1.74 with every drift general, 0.66 without a bound).
+// 2.53 ms (1.74 with every drift general, 0.72 without a bound).
 constexpr float TINY_DRIFT_TH = 0x1p-34f, FAR_DRIFT_TH = 0x1p-110f;
 
 // --- float-float without the renormalising step: hi + lo with |lo| up to a
@@ -330,9 +335,10 @@ __device__ __forceinline__ float kepler_residual(ff X, ff Y, float w, ff q2, ff 
 // the ensembles 5 %.  The line at 1e-2: e, q2 and q3 at 2^-46 then change
 // r by 2^-55 and v by 2^-53 at most, and the series end below 2^-46.  300,000
 // scattered-disk particles x 256 steps, 0.9 % of their drifts here and 0.1 % beyond,
-// but spread over the warps: 7.19 -> 6.47 ms (5.15 with tau^2 / 2 down to 2^-34), error against long double 3.1e-15 before
-// and after; 1e6 particles x 64 steps with the learned starter
-// 5.94 -> 5.21 ms.
+// but spread over the warps: 7.19 -> 6.47 ms (5.15 with tau^2 / 2 down to 2^-34; 5.31
+// since the conversions tell both ends of their range and zero apart), error against
+// long double 3.1e-15 before and after; 1e6 particles x 64 steps with the learned
+// starter 5.94 -> 5.21 ms.
 template <bool MEDIUM>
 __device__ __forceinline__ int small_drift(ff rx, ff ry, ff rz, ff vx, ff vy, ff vz, ff r2, ff rinv, ff muh, ff mudt,
                                            const SmallStepDt& c, SmallDrift& d)

@@ -61,7 +61,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, CTAS_PER_SM)
 // runs a grid that it takes in fewer waves: a wave of a few CTAs lasts as long as
 // their serial chain.  100,000 close-eccentric particles x 128 steps (one wave of
 // either) 3.40 ms with 14 CTAs and 4.44 with 16, 135,000 4.12 and 4.49, 140,000 (two
-// waves of 14) 5.34 and 4.58, 150,000 5.70 and 4.83.
+// waves of 14) 5.34 and 4.58, 150,000 5.70 and 4.83.  With many waves it matters little
+// which runs, and 16, which the rule then takes, is not always the faster: 1e6
+// particles x 64 steps 14.66 ms against 14.46 with 14 where every drift takes the
+// network, 5.15 against 5.31 on the scattered disk.
 inline bool learned_saves_a_wave(uint32_t grid, uint32_t sms)
 {
     const uint32_t lean = sms * GLISSER_TB_MIN_BLOCKS_LEARNED, full = sms * GLISSER_TB_MIN_BLOCKS;

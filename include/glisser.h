@@ -49,7 +49,8 @@ extern "C" {
 /* Kepler starters for the universal-variable drift. */
 #define GLISSER_STARTER_CLASSIC 0  /* the reference's kepu_guess, src/wh.cpp:188-220 */
 #define GLISSER_STARTER_SERIES 1   /* tenth-order time series / FP32 Kepler pre-solve */
-#define GLISSER_STARTER_LEARNED 2  /* series where it applies, else the MLP initial guess; classic fallback */
+#define GLISSER_STARTER_LEARNED 2  /* series where it applies, else the MLP initial guess; classic fallback.
+                                      SERIES is the faster choice on every workload measured */
 
 /* What the time-block kernel does with a particle that ends the block in a
  * close encounter (flags != 0, (flags & 0xFE) == 0), glisser_step_params
@@ -60,9 +61,15 @@ extern "C" {
                                           SWIFT hand-off resumes from (src/executor.cu:624-633, 827-834) */
 
 /* Arithmetic of the planet kick and its radius tests (glisser_step_params
- * .kick).  The reference computes them in FP64 (src/wh.cu:142-172). */
-#define GLISSER_KICK_FLOAT_FLOAT 0  /* default: float-float (~48 bits) on the FP32 pipe; the drift stays FP64 */
-#define GLISSER_KICK_FP64 1         /* FP64, the reference's formulation */
+ * .kick).  The reference computes them in FP64 (src/wh.cu:142-172).  The choice
+ * does not extend to the drift, which is the same with both: positions and
+ * velocities are FP64, and what a step adds to them is formed in FP64 for a drift
+ * with tau^2 = dt^2 mu / r^3 >= 1e-3, with an FP32 start, and in float-float below,
+ * where the correction is small next to the state (errors against long double
+ * no larger than with FP64 throughout).  GLISSER_STARTER_CLASSIC runs every
+ * drift in FP64. */
+#define GLISSER_KICK_FLOAT_FLOAT 0  /* default: float-float (~48 bits) on the FP32 pipe */
+#define GLISSER_KICK_FP64 1         /* FP64, the reference's formulation of the kick */
 
 /* Feature normalisation and training box of a learned starter (features
  * f0 = log(tau), tau = dt sqrt(mu/r0^3), f1 = r0.v0 / sqrt(mu r0),
@@ -112,7 +119,8 @@ typedef struct glisser_step_params {
     int32_t starter;             /* GLISSER_STARTER_* */
     int32_t kill_encounters;     /* GLISSER_ENCOUNTERS_*: what a particle flagged 0x01 keeps */
     const void *mlp;             /* learned-starter weights (device), or NULL */
-    double kepler_tol;           /* Kepler residual tolerance |f| < tol*dt; 0 = 1e-13 (the reference's DANBYB) */
+    double kepler_tol;           /* Kepler residual tolerance |f| < tol*dt; 0 = 1e-13 (the reference's DANBYB);
+                                    see glisser_set_kepler_tolerance */
     int32_t kick;                /* GLISSER_KICK_*: arithmetic of the planet kick and its radius tests */
     int32_t reserved;
 } glisser_step_params;
@@ -222,7 +230,9 @@ int glisser_set_device_interp(glisser_t *h, int on);
 /* Kepler residual tolerance of the drift's Newton iteration, |f| < tol * dt
  * (the reference's DANBYB is 1e-13, the default); 1e-16 <= tol <= 1e-8.  The
  * accepted Newton correction is folded into the G-functions, so the solution
- * error is O(tol^2). */
+ * error is O(tol^2).  It applies to the drifts that iterate in FP64: bound orbits
+ * with tau^2 = dt^2 mu / r^3 below 1e-2 (series and learned starters) are solved in
+ * float-float to the state's own FP64 rounding whatever the tolerance. */
 int glisser_set_kepler_tolerance(glisser_t *h, double tol);
 
 /* Arithmetic of the planet kick and its radius tests: GLISSER_KICK_FLOAT_FLOAT
